@@ -358,7 +358,7 @@ size_t scratch_need(const Work& w, long long cnt)
     long long g = (long long)(cap / one);
     if (g < 1) g = 1;
     if (g > cnt) g = cnt;
-    return one * (size_t)g;
+    return one * (size_t)g + (is_real(w.kind) ? 0 : ckg::flow_scratch_extra(w.log2n, g));
 }
 
 // Whether kernels reading and writing page-locked host memory in place beat

@@ -93,18 +93,23 @@ __device__ __forceinline__ float2 rot(float2 a)
     }
 }
 
-// ------------------------------------------------------- in-register DFTs
+// a + i b and a - i b.
+__device__ __forceinline__ float2 cadd_i(float2 a, float2 b) { return make_float2(a.x - b.y, a.y + b.x); }
+__device__ __forceinline__ float2 csub_i(float2 a, float2 b) { return make_float2(a.x + b.y, a.y - b.x); }
 
-template <int R, bool INV> __device__ __forceinline__ void dft(float2 (&v)[R]);
+// ------------------------------------------------------- in-register DFTs
+// V: one complex value (float2), or two packed ones (cpair, fft_pair.cuh).
+
+template <int R, bool INV, class V> __device__ __forceinline__ void dft(V (&v)[R]);
 
 // Cooley-Tukey split R = P*Q on registers: n = Q*n1 + n2, k = k1 + P*k2.
-template <int R, int P, bool INV>
-__device__ __forceinline__ void dft_ct(float2 (&v)[R])
+template <int R, int P, bool INV, class V>
+__device__ __forceinline__ void dft_ct(V (&v)[R])
 {
     constexpr int Q = R / P;
     static_for<0, Q>([&](auto n2c) {
         constexpr int n2 = decltype(n2c)::value;
-        float2 t[P];
+        V t[P];
 #pragma unroll
         for (int n1 = 0; n1 < P; ++n1) t[n1] = v[Q * n1 + n2];
         dft<P, INV>(t);
@@ -113,10 +118,10 @@ __device__ __forceinline__ void dft_ct(float2 (&v)[R])
             v[Q * k1 + n2] = rot<R, n2 * k1, INV>(t[k1]);
         });
     });
-    float2 o[R];
+    V o[R];
 #pragma unroll
     for (int k1 = 0; k1 < P; ++k1) {
-        float2 t[Q];
+        V t[Q];
 #pragma unroll
         for (int n2 = 0; n2 < Q; ++n2) t[n2] = v[Q * k1 + n2];
         dft<Q, INV>(t);
@@ -127,26 +132,26 @@ __device__ __forceinline__ void dft_ct(float2 (&v)[R])
     for (int k = 0; k < R; ++k) v[k] = o[k];
 }
 
-template <int R, bool INV>
-__device__ __forceinline__ void dft(float2 (&v)[R])
+template <int R, bool INV, class V>
+__device__ __forceinline__ void dft(V (&v)[R])
 {
     if constexpr (R == 1) {
         (void)v;
     } else if constexpr (R == 2) {
-        float2 a = v[0], b = v[1];
+        V a = v[0], b = v[1];
         v[0] = cadd(a, b);
         v[1] = csub(a, b);
     } else if constexpr (R == 4) {
-        float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-        float2 a2 = cadd(v[1], v[3]), a3 = csub(v[1], v[3]);
+        V a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
+        V a2 = cadd(v[1], v[3]), a3 = csub(v[1], v[3]);
         v[0] = cadd(a0, a2);
         v[2] = csub(a0, a2);
         if (INV) {
-            v[1] = make_float2(a1.x - a3.y, a1.y + a3.x);
-            v[3] = make_float2(a1.x + a3.y, a1.y - a3.x);
+            v[1] = cadd_i(a1, a3);
+            v[3] = csub_i(a1, a3);
         } else {
-            v[1] = make_float2(a1.x + a3.y, a1.y - a3.x);
-            v[3] = make_float2(a1.x - a3.y, a1.y + a3.x);
+            v[1] = csub_i(a1, a3);
+            v[3] = cadd_i(a1, a3);
         }
     } else if constexpr (R == 8) {
         dft_ct<8, 2, INV>(v);
@@ -222,10 +227,14 @@ __device__ __forceinline__ void xsync()
 // until the previous one has completed and its writes are visible, before
 // any memory access.  After a kernel that never signals, the wait returns at
 // once: the launch then behaves like a plain one.
+// A kernel may split the two to read memory that no kernel writes (the twiddle
+// table) before the wait.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_start()
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch_dependents();
+    pdl_wait();
 }
 
 // ------------------------------------------------------- Stockham engine

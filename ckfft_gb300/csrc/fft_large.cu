@@ -336,7 +336,13 @@ cudaError_t launch_large_c2c(bool inverse, int log2n, const void* in, void* out,
                                  group, s);
     for (long long off = 0; off < count; off += group) {
         const long long cnt = count - off < group ? count - off : group;
-        cudaError_t e = inverse
+        cudaError_t e = cudaSuccess;
+        if (launch_flow(inverse, log2n, src + off * in_dist, dst + off * out_dist, cnt, in_dist, out_dist, tw, tmp,
+                        scratch_bytes, s, &e)) {
+            if (e != cudaSuccess) return e;
+            continue;
+        }
+        e = inverse
             ? launch_cols<true>(p.log2n1, src + off * in_dist, tmp, cnt, p.log2n2, in_dist, n, tw, s)
             : launch_cols<false>(p.log2n1, src + off * in_dist, tmp, cnt, p.log2n2, in_dist, n, tw, s);
         if (e != cudaSuccess) return e;

@@ -120,6 +120,16 @@ cudaError_t launch_l2pass(int kind, int log2n, const void* in, void* out, long l
                           long long out_dist, const float2* tw, void* scratch, size_t scratch_bytes,
                           cudaStream_t stream);
 
+// Both passes of a batch of complex 2^17 .. 2^20 transforms in one launch with
+// the intermediates in L2 (fft_flow.cu).  False (nothing launched) where it
+// does not apply: other sizes, too little work, data that TMA cannot address
+// (not 16-byte aligned), a scratch block without flow_scratch_extra() bytes
+// behind the intermediates.
+size_t flow_scratch_extra(int log2n, long long count);
+bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long count, long long in_dist,
+                 long long out_dist, const float2* tw, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                 cudaError_t* e);
+
 // Complex 2^15 and 2^16 on persistent CTAs, one transform per CTA at a time,
 // both passes inside the CTA with bulk-copied tiles and the intermediate in
 // L2 (fft_mid.cu).  scratch: mid_scratch_bytes(), 128-byte aligned; in
