@@ -231,6 +231,14 @@ __device__ __forceinline__ void xsync()
 // table) before the wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel let in only once this one's wait is over: a kernel of few
+// CTAs that runs in one wave then does not share its SMs with the next one's
+// waiting CTAs (one 2^20 transform, two passes: 15.8 -> 10.1 us).
+__device__ __forceinline__ void pdl_wait_then_launch()
+{
+    pdl_wait();
+    pdl_launch_dependents();
+}
 __device__ __forceinline__ void pdl_start()
 {
     pdl_launch_dependents();

@@ -10,14 +10,14 @@
 //                     transposed through shared memory.
 //
 // Both passes read and write HBM once, with C adjacent columns (pass 1) or
-// rows (pass 2) per CTA so every warp access covers C*8 contiguous bytes.
+// rows (pass 2) per CTA so every warp access covers C*8 contiguous bytes
+// (large batches of complex 2^17 .. 2^20: fft_flow.cu).
 // Real sizes run the half-length complex transform with the split (forward)
 // fused into its last pass and the merge (inverse) into its first, the
-// algebra of src/ckfft/fft_real_default.cpp; a separate split / merge kernel
-// remains for scratch arrays that are not 128-byte aligned.
+// algebra of src/ckfft/fft_real_default.cpp.
 #include <cstdint>
 
-#include "fft_passes.cuh"
+#include "fft_pair_passes.cuh"
 #include "jobs.h"
 #include "kernels.h"
 
@@ -25,56 +25,38 @@ namespace ckg {
 
 // ------------------------------------------------------------ pass kernels
 
-// Thread budget of the batched pass kernels: 1024 for sub-lengths above 2^10
-// (16 values per thread, 64 registers), 512 below.
+// Tiles of 16 columns or rows (128-byte row accesses), 8 at sub-length 2^10,
+// two columns or rows a thread (fft_pair_passes.cuh), at most 256 threads and
+// 128 registers a thread.
 template <int LS>
-struct BatchMaxT {
-    static constexpr int value = LS > 10 ? 1024 : 512;
-};
-// Widest tile of the batched passes: 16 sequences (128-byte row accesses).
-// 32 (256-byte rows) up to sub-length 2^8 measured slower on GB300: batched
-// 2^17 2604 vs 2740 GB/s, 2^24 1723 vs 1942 (twice the shared memory per
-// CTA, half the CTAs per SM).
+using BPass = PairCfg<LS, 256, 8>;
 template <int LS>
-struct BatchCMax {
-    static constexpr int value = 16;
-};
-template <int LS>
-using BPass = PassCfg<LS, BatchMaxT<LS>::value, BatchCMax<LS>::value>;
-// Resident CTAs asked of the compiler for the column kernels: at most 64
-// registers a thread, so that at sub-lengths 2^9 / 2^10 (512 threads) two
-// CTAs share an SM and one's loads overlap the other's butterflies.
-template <int LS>
-struct ColsMinBlocks {
-    static constexpr int value = 65536 / (BPass<LS>::THREADS * 64);
-};
+constexpr int kPassBlocks = 65536 / (BPass<LS>::THREADS * 128);
 
 template <int LA, bool INV>
-__global__ void __launch_bounds__(BPass<LA>::THREADS, ColsMinBlocks<LA>::value)
-k_cols(const float2* __restrict__ in, float2* __restrict__ out, long long count, int log2n2,
-       long long in_dist, long long out_dist, const float2* __restrict__ tw)
+__global__ void __launch_bounds__(BPass<LA>::THREADS, kPassBlocks<LA>)
+k_cols(const float2* __restrict__ in, float2* __restrict__ out, int log2n2, long long in_dist, long long out_dist,
+       const float2* __restrict__ tw)
 {
     using P = BPass<LA>;
-    extern __shared__ float2 smem[];
-    pdl_start();
-    const long long tiles = (1ll << log2n2) / P::C;
-    const long long f = blockIdx.x / tiles;
-    pass_cols<LA, INV, false, BatchMaxT<LA>::value, BatchCMax<LA>::value>(in + f * in_dist, out + f * out_dist, log2n2,
-                                                                          blockIdx.x % tiles, threadIdx.x, smem, tw);
+    extern __shared__ __align__(128) cpair smem[];
+    const int log2tiles = log2n2 - ilog2(P::C);
+    const long long f = blockIdx.x >> log2tiles;
+    pair_cols<LA, INV, P>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
+                          smem, tw, [] { pdl_wait_then_launch(); });
 }
 
 template <int LB, bool INV>
-__global__ void __launch_bounds__(BPass<LB>::THREADS)
-k_rows(const float2* __restrict__ in, float2* __restrict__ out, long long count, int log2n1,
-       long long in_dist, long long out_dist, const float2* __restrict__ tw)
+__global__ void __launch_bounds__(BPass<LB>::THREADS, kPassBlocks<LB>)
+k_rows(const float2* __restrict__ in, float2* __restrict__ out, int log2n1, long long in_dist, long long out_dist,
+       const float2* __restrict__ tw)
 {
     using P = BPass<LB>;
-    extern __shared__ float2 smem[];
-    pdl_start();
-    const long long tiles = (1ll << log2n1) / P::C;
-    const long long f = blockIdx.x / tiles;
-    pass_rows_xt<LB, INV, false, BatchMaxT<LB>::value, true, BatchCMax<LB>::value>(
-        in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x % tiles, threadIdx.x, smem, tw);
+    extern __shared__ __align__(128) cpair smem[];
+    const int log2tiles = log2n1 - ilog2(P::C);
+    const long long f = blockIdx.x >> log2tiles;
+    pair_rows<LB, INV, P>(in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
+                          smem, tw, LB, [] { pdl_wait_then_launch(); });
 }
 
 // Third pass of the three-pass transform (N = N1 N2 N3, sub-lengths 2^l1,
@@ -82,82 +64,62 @@ k_rows(const float2* __restrict__ in, float2* __restrict__ out, long long count,
 // tile, row (k1, k2) of transform f at in[f N + k1 N2 N3 + k2 N3 ..], and
 // stores X[k1 + N1 k2 + N1 N2 k3] -- C consecutive outputs per k3.
 template <int LB, bool INV>
-__global__ void __launch_bounds__(BPass<LB>::THREADS)
+__global__ void __launch_bounds__(BPass<LB>::THREADS, kPassBlocks<LB>)
 k_rows3(const float2* __restrict__ in, float2* __restrict__ out, int l1, int l2, long long out_dist,
         const float2* __restrict__ tw)
 {
     using P = BPass<LB>;
-    extern __shared__ float2 smem[];
-    pdl_start();
-    const long long tiles = (1ll << l1) / P::C;
+    extern __shared__ __align__(128) cpair smem[];
+    const int log2tiles = l1 - ilog2(P::C);
     const long long b = blockIdx.x;
-    const long long tile = b % tiles;
-    const long long k2 = (b / tiles) & ((1ll << l2) - 1);
-    const long long f = b / (tiles << l2);
+    const int tile = (int)(b & ((1 << log2tiles) - 1));
+    const long long k2 = (b >> log2tiles) & ((1ll << l2) - 1);
+    const long long f = b >> (log2tiles + l2);
     const long long n = 1ll << (l1 + l2 + LB);
-    pass_rows_xt<LB, INV, false, BatchMaxT<LB>::value, true, BatchCMax<LB>::value>(
-        in + f * n + (k2 << LB), out + f * out_dist + (k2 << l1), l1 + l2, tile, threadIdx.x, smem, tw, l2 + LB);
+    pair_rows<LB, INV, P>(in + f * n + (k2 << LB), out + f * out_dist + (k2 << l1), l1 + l2, tile, threadIdx.x, smem, tw,
+                          l2 + LB, [] { pdl_wait_then_launch(); });
 }
+
+// The split and merge passes run one value a thread (fft_passes.cuh), 512
+// threads and 64 registers: two values a thread measured slower there, more so
+// with other streams' kernels (real 2^18 x 127 forward 111 -> 114 us, a pair on
+// three streams 207 -> 218; 2^21 x 16 inverse 155 -> 163): the mirrored halves
+// leave stores of 8 bytes and loads of single bins, which want warps in flight.
+template <int LS>
+using SPass = PassCfg<LS, 512>;
+template <int LS>
+constexpr int kSplitBlocks = 65536 / (SPass<LS>::THREADS * 64);
 
 // Row pass of a real forward transform with the split fused: block
 // (f, tile) writes the M+1 output bins of its row pairs (pass_rows_split).
 template <int LB>
-__global__ void __launch_bounds__(BPass<LB>::THREADS)
+__global__ void __launch_bounds__(SPass<LB>::THREADS, kSplitBlocks<LB>)
 k_rows_split(const float2* __restrict__ in, float2* __restrict__ out, int log2n1, int log2k1, long long in_dist,
              long long out_dist, const float2* __restrict__ tw)
 {
-    using P = BPass<LB>;
-    extern __shared__ float2 smem[];
-    pdl_start();
-    const long long tiles = (1ll << log2n1) / P::C;
-    const long long f = blockIdx.x / tiles;
-    pass_rows_split<LB, BatchMaxT<LB>::value>(in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x % tiles,
-                                              threadIdx.x, smem, tw, log2k1);
+    using P = SPass<LB>;
+    extern __shared__ __align__(128) float2 smem1[];
+    pdl_wait_then_launch();
+    const int log2tiles = log2n1 - ilog2(P::C);
+    const long long f = blockIdx.x >> log2tiles;
+    pass_rows_split<LB, 512>(in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x & ((1 << log2tiles) - 1),
+                             threadIdx.x, smem1, tw, log2k1);
 }
 
 // Column pass of a real inverse transform with the merge fused: block
 // (f, tile) reads the M+1 bins of its column pairs (pass_cols_merge).
 template <int LA>
-__global__ void __launch_bounds__(BPass<LA>::THREADS, ColsMinBlocks<LA>::value)
+__global__ void __launch_bounds__(SPass<LA>::THREADS, kSplitBlocks<LA>)
 k_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2, long long in_dist,
              long long out_dist, const float2* __restrict__ tw)
 {
-    using P = BPass<LA>;
-    extern __shared__ float2 smem[];
-    pdl_start();
-    const long long tiles = (1ll << log2n2) / P::C;
-    const long long f = blockIdx.x / tiles;
-    pass_cols_merge<LA, BatchMaxT<LA>::value, BatchCMax<LA>::value>(in + f * in_dist, out + f * out_dist, log2n2,
-                                                                    blockIdx.x % tiles, threadIdx.x, smem, tw);
-}
-
-// --------------------------- real split / merge as passes of their own
-// (used only when the scratch array is not 128-byte aligned)
-
-// In-place split of a natural-order half-length spectrum Z (M = 2^lm values,
-// with room for M+1) into the real forward output X[0..M].
-__global__ void k_split_inplace(float2* __restrict__ z, long long count, int lm, long long dist,
-                                const float2* __restrict__ tw)
-{
-    pdl_start();
-    const long long M = 1ll << lm;
-    const long long per = M / 2 + 1;                 // pairs (k, M-k) for k = 0..M/2
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= count * per) return;
-    const long long f = idx / per, k = idx % per;
-    split_pair_inplace<false>(z + f * dist, M, k, tw + 2 * M);
-}
-
-// Y[k] = merge(X[k], X[M-k]) for k < M, written as M complex values.
-__global__ void k_merge(const float2* __restrict__ x, float2* __restrict__ y, long long count, int lm,
-                        long long in_dist, long long out_dist, const float2* __restrict__ tw)
-{
-    pdl_start();
-    const long long M = 1ll << lm;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= count * M) return;
-    const long long f = idx >> lm, k = idx & (M - 1);
-    merge_elem<false>(x + f * in_dist, y + f * out_dist, M, k, tw + 2 * M);
+    using P = SPass<LA>;
+    extern __shared__ __align__(128) float2 smem1[];
+    pdl_wait_then_launch();
+    const int log2tiles = log2n2 - ilog2(P::C);
+    const long long f = blockIdx.x >> log2tiles;
+    pass_cols_merge<LA, 512>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1),
+                             threadIdx.x, smem1, tw);
 }
 
 // ---------------------------------------------------------------- launch
@@ -168,8 +130,8 @@ static cudaError_t launch_cols_L(const float2* in, float2* out, long long count,
 {
     using P = BPass<LA>;
     const long long blocks = count * ((1ll << log2n2) / P::C);
-    return launch_pdl(k_cols<LA, INV>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, count, log2n2,
-                      in_dist, out_dist, tw);
+    return launch_pdl(k_cols<LA, INV>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n2, in_dist,
+                      out_dist, tw);
 }
 
 template <int LB, bool INV>
@@ -178,8 +140,8 @@ static cudaError_t launch_rows_L(const float2* in, float2* out, long long count,
 {
     using P = BPass<LB>;
     const long long blocks = count * ((1ll << log2n1) / P::C);
-    return launch_pdl(k_rows<LB, INV>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, count, log2n1,
-                      in_dist, out_dist, tw);
+    return launch_pdl(k_rows<LB, INV>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n1, in_dist,
+                      out_dist, tw);
 }
 
 #define CKG_SUB_SWITCH(L, FN, ...)                                                                 \
@@ -188,10 +150,6 @@ static cudaError_t launch_rows_L(const float2* in, float2* out, long long count,
     case 8: return FN<8, INV>(__VA_ARGS__);                                                        \
     case 9: return FN<9, INV>(__VA_ARGS__);                                                        \
     case 10: return FN<10, INV>(__VA_ARGS__);                                                      \
-    case 11: return FN<11, INV>(__VA_ARGS__);                                                      \
-    case 12: return FN<12, INV>(__VA_ARGS__);                                                      \
-    case 13: return FN<13, INV>(__VA_ARGS__);                                                      \
-    case 14: return FN<14, INV>(__VA_ARGS__);                                                      \
     default: return cudaErrorInvalidValue;                                                         \
     }
 
@@ -276,6 +234,7 @@ static cudaError_t launch_three_pass(Kind kind, int log2n, const float2* in, flo
         if (e == cudaSuccess)
             e = inverse ? launch_cols<true>(l2, tmp, tmp, cnt << l1, l3, M, M, tw, s)
                         : launch_cols<false>(l2, tmp, tmp, cnt << l1, l3, M, M, tw, s);
+        count_launch(2);
         // pass 3: rows of length N3, C consecutive k1 per tile -> out (real
         // forward: row pairs k, N1 N2 - k with the split)
         if (e == cudaSuccess)
@@ -283,7 +242,7 @@ static cudaError_t launch_three_pass(Kind kind, int log2n, const float2* in, flo
                 : inverse   ? launch_rows3<true>(l3, tmp, dst, cnt, l1, l2, out_dist, tw, s)
                             : launch_rows3<false>(l3, tmp, dst, cnt, l1, l2, out_dist, tw, s);
         if (e != cudaSuccess) return e;
-        count_launch(3);
+        count_launch();
     }
     return cudaSuccess;
 }
@@ -314,15 +273,16 @@ cudaError_t launch_large_c2c(bool inverse, int log2n, const void* in, void* out,
                              long long in_dist, long long out_dist, const float2* tw,
                              void* scratch, size_t scratch_bytes, cudaStream_t s)
 {
-    if (!large_supported(log2n)) return cudaErrorInvalidValue;
+    // the row passes drop the intermediate's 128-byte L2 lines
+    if (!large_supported(log2n) || ((uintptr_t)scratch & 127)) return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
     // 2^15, 2^16: both passes inside one persistent CTA per transform
     // (fft_mid.cu), or inside one cluster per transform (fft_l2pass.cu); the
     // intermediate kept in L2 either way
-    if (mid_supported(log2n) && mid_enabled(log2n) && ((uintptr_t)scratch & 127) == 0 && ((uintptr_t)in & 15) == 0 &&
+    if (mid_supported(log2n) && mid_enabled(log2n) && ((uintptr_t)in & 15) == 0 &&
         (in_dist & 1) == 0 && scratch_bytes >= mid_scratch_bytes(log2n, count))
         return launch_mid(inverse ? 1 : 0, log2n, in, out, count, in_dist, out_dist, tw, scratch, scratch_bytes, s);
-    if (l2pass_supported(log2n) && ((uintptr_t)scratch & 127) == 0)
+    if (l2pass_supported(log2n))
         return launch_l2pass(inverse ? 1 : 0, log2n, in, out, count, in_dist, out_dist, tw, scratch, scratch_bytes, s);
     const LargePlan p = large_plan(log2n);
     const long long n = 1ll << log2n;
@@ -331,7 +291,7 @@ cudaError_t launch_large_c2c(bool inverse, int log2n, const void* in, void* out,
     const float2* src = (const float2*)in;
     float2* dst = (float2*)out;
     float2* tmp = (float2*)scratch;
-    if (log2n >= kThreePassMinLog2 && ((uintptr_t)scratch & 127) == 0)
+    if (log2n >= kThreePassMinLog2)
         return launch_three_pass(inverse ? C2C_INV : C2C_FWD, log2n, src, dst, count, in_dist, out_dist, tw, tmp,
                                  group, s);
     for (long long off = 0; off < count; off += group) {
@@ -359,7 +319,7 @@ template <int LB>
 static cudaError_t launch_rows_split_L(const float2* in, float2* out, long long count, int log2n1, int log2k1,
                                        long long in_dist, long long out_dist, const float2* tw, cudaStream_t s)
 {
-    using P = BPass<LB>;
+    using P = SPass<LB>;
     const long long blocks = count * ((1ll << log2n1) / P::C);
     return launch_pdl(k_rows_split<LB>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n1,
                       log2k1, in_dist, out_dist, tw);
@@ -415,35 +375,28 @@ cudaError_t launch_large_r2c(int log2n, const void* in, void* out, long long cou
     // / 2609 for the fused two-pass form through HBM)
     const int lm = log2n - 1;
     const long long M = 1ll << lm;
+    if ((uintptr_t)scratch & 127) return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
-    if (l2pass_supported(lm) && ((uintptr_t)scratch & 127) == 0)
+    if (l2pass_supported(lm))
         return launch_l2pass(2, lm, in, out, count, in_dist / 2, out_dist, tw, scratch, scratch_bytes, s);
-    if (rows_split_supported(lm) && ((uintptr_t)scratch & 127) == 0)
+    if (rows_split_supported(lm))
         return launch_r2c_rows_split(lm, (const float2*)in, (float2*)out, count, in_dist / 2, out_dist, tw,
                                      (float2*)scratch, scratch_bytes, s);
     int l1, l2, l3;
-    if (lm >= kThreePassMinLog2 && plan3(lm, &l1, &l2, &l3) && ((uintptr_t)scratch & 127) == 0) {
+    if (lm >= kThreePassMinLog2 && plan3(lm, &l1, &l2, &l3)) {
         const long long group = (long long)(scratch_bytes / (sizeof(float2) * (size_t)M));
         if (group < 1) return cudaErrorInvalidValue;
         return launch_three_pass(R2C, lm, (const float2*)in, (float2*)out, count, in_dist / 2, out_dist, tw,
                                  (float2*)scratch, group, s);
     }
-    cudaError_t e = launch_large_c2c(false, lm, in, out, count, in_dist / 2, out_dist, tw, scratch,
-                                     scratch_bytes, s);
-    if (e != cudaSuccess) return e;
-    const long long work = count * (M / 2 + 1);
-    const int threads = 256;
-    e = launch_pdl(k_split_inplace, dim3((unsigned)((work + threads - 1) / threads)), dim3(threads), 0, s,
-                   (float2*)out, count, lm, out_dist, tw);
-    count_launch();
-    return e;
+    return cudaErrorInvalidValue;
 }
 
 template <int LA>
 static cudaError_t launch_cols_merge_L(const float2* in, float2* out, long long count, int log2n2,
                                        long long in_dist, long long out_dist, const float2* tw, cudaStream_t s)
 {
-    using P = BPass<LA>;
+    using P = SPass<LA>;
     const long long blocks = count * ((1ll << log2n2) / P::C);
     return launch_pdl(k_cols_merge<LA>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n2,
                       in_dist, out_dist, tw);
@@ -500,62 +453,44 @@ cudaError_t launch_large_c2r(int log2n, const void* in, void* out, long long cou
     // 2714 / 2554 for the fused two-pass form through HBM)
     const int lm = log2n - 1;
     const long long M = 1ll << lm;
+    if ((uintptr_t)scratch & 127) return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
-    if (l2pass_supported(lm) && ((uintptr_t)scratch & 127) == 0)
+    if (l2pass_supported(lm))
         return launch_l2pass(3, lm, in, out, count, in_dist, out_dist / 2, tw, scratch, scratch_bytes, s);
-    if (cols_merge_supported(lm) && ((uintptr_t)scratch & 127) == 0)
+    if (cols_merge_supported(lm))
         return launch_c2r_cols_merge(lm, (const float2*)in, (float2*)out, count, in_dist, out_dist / 2, tw,
                                      (float2*)scratch, scratch_bytes, s);
     int l1, l2, l3;
-    if (lm >= kThreePassMinLog2 && plan3(lm, &l1, &l2, &l3) && ((uintptr_t)scratch & 127) == 0) {
+    if (lm >= kThreePassMinLog2 && plan3(lm, &l1, &l2, &l3)) {
         const long long group = (long long)(scratch_bytes / (sizeof(float2) * (size_t)M));
         if (group < 1) return cudaErrorInvalidValue;
         return launch_three_pass(C2R, lm, (const float2*)in, (float2*)out, count, in_dist, out_dist / 2, tw,
                                  (float2*)scratch, group, s);
     }
-    const long long work = count * M;
-    const int threads = 256;
-    cudaError_t e = launch_pdl(k_merge, dim3((unsigned)((work + threads - 1) / threads)), dim3(threads), 0, s,
-                               (const float2*)in, (float2*)out, count, lm, in_dist, out_dist / 2, tw);
-    count_launch();
-    if (e != cudaSuccess) return e;
-    // inverse complex transform of the merged values, in place through scratch
-    return launch_large_c2c(true, lm, out, out, count, out_dist / 2, out_dist / 2, tw, scratch,
-                            scratch_bytes, s);
+    return cudaErrorInvalidValue;
 }
 
 template <int L>
 static cudaError_t attr_pass()
 {
-    using P = BPass<L>;
-    cudaError_t e;
-    if constexpr (L <= 10) {
-        if ((e = cudaFuncSetAttribute(k_rows3<L, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-        if ((e = cudaFuncSetAttribute(k_rows3<L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    }
-    if constexpr (L >= 7 && L <= 10) {
-        if ((e = cudaFuncSetAttribute(k_rows_split<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    }
-    if constexpr (L >= 7 && L <= 10) {
-        if ((e = cudaFuncSetAttribute(k_cols_merge<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    }
-    if ((e = cudaFuncSetAttribute(k_cols<L, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_cols<L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_rows<L, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_rows<L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM);
+    const int smem = (int)BPass<L>::SMEM;
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_rows3<L, false>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows3<L, true>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows_split<L>, a, (int)SPass<L>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols_merge<L>, a, (int)SPass<L>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, false>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, true>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows<L, false>, a, smem);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k_rows<L, true>, a, smem) : e;
 }
 
 cudaError_t prepare_large()
 {
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = attr_pass<7>();
+    cudaError_t e = attr_pass<7>();
     if (e == cudaSuccess) e = attr_pass<8>();
     if (e == cudaSuccess) e = attr_pass<9>();
     if (e == cudaSuccess) e = attr_pass<10>();
-    if (e == cudaSuccess) e = attr_pass<11>();
-    if (e == cudaSuccess) e = attr_pass<12>();
-    if (e == cudaSuccess) e = attr_pass<13>();
-    if (e == cudaSuccess) e = attr_pass<14>();
     return e;
 }
 

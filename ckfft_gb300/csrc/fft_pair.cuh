@@ -121,25 +121,6 @@ __device__ __forceinline__ cpair rot(cpair a)
     }
 }
 
-// real_split / real_merge of fft_core.cuh on both lanes, a twiddle per lane.
-__device__ __forceinline__ cpair real_split(cpair z0, cpair z1, cpair w)
-{
-    const f32x2 sx = add2(z0.x, z1.x), sy = sub2(z0.y, z1.y);
-    const f32x2 dx = sub2(z0.x, z1.x), dy = add2(z0.y, z1.y);
-    const f32x2 ny = neg2(w.y);
-    const f32x2 cx = fma2(ny, dx, neg2(mul2(w.x, dy)));
-    const f32x2 cy = fma2(w.x, dx, mul2(ny, dy));
-    return {sub2(sx, cx), sub2(sy, cy)};
-}
-__device__ __forceinline__ cpair real_merge(cpair z0, cpair z1, cpair w)
-{
-    const f32x2 sx = add2(z0.x, z1.x), sy = sub2(z0.y, z1.y);
-    const f32x2 dx = sub2(z0.x, z1.x), dy = add2(z0.y, z1.y);
-    const f32x2 cx = fma2(w.y, dx, neg2(mul2(w.x, dy)));
-    const f32x2 cy = fma2(w.x, dx, mul2(w.y, dy));
-    return {add2(sx, cx), add2(sy, cy)};
-}
-
 // ------------------------------------------------------------ shared memory
 // Position pos of the transform pair a view belongs to, at
 // base[(PAD ? pos + pos / 16 : pos) * MUL]: a tile of MUL pairs side by side
@@ -157,7 +138,7 @@ struct PairView {
 };
 
 // Where a stage's table twiddles come from: element k of level 2^q (W_{2^q}^k,
-// conjugated for the inverse).  StageTable: a copy of the levels a transform
+// conjugated for the inverse), for the thread's butterfly u.  StageTable: a copy of the levels a transform
 // of 2^LS points (16 values a thread) uses, in shared memory, so that no
 // stage waits for L2.
 template <int LS, bool INV>
@@ -172,7 +153,7 @@ struct StageTable {
         else if constexpr (LEVEL == 1024) return 64 + k;                   // k < 256
         else return 64 + (LS == 10 ? 256 : 0) + k;                         // 512
     }
-    template <int LEVEL>
+    template <int LEVEL, int U>
     __device__ __forceinline__ float2 get(int k) const { return s[at<LEVEL>(k)]; }
     // fills the copy from the table of all levels, by threads tid of `threads`
     __device__ static void fill(float2* d, const float2* __restrict__ tw, int tid, int threads)
@@ -187,6 +168,42 @@ struct StageTable {
         level(std::integral_constant<int, 256>{}, 16);
         if constexpr (LS >= 9) level(std::integral_constant<int, 512>{}, 256);
         if constexpr (LS == 10) level(std::integral_constant<int, 1024>{}, 256);
+    }
+};
+
+// The same twiddles of one thread in registers, for a kernel that runs each
+// stage once a thread: all of them are loaded before the thread's data (and
+// before the wait for the previous kernel), so no stage waits for them.
+// Second stage (span 16, radix RS2) at thread position t2, third (span 256)
+// at t3 (the row passes' last stage runs on other positions).
+template <int LS, bool INV>
+struct StageRegs {
+    using S = Sched<LS, 4>;
+    static constexpr int T = (1 << LS) / 16;
+    static constexpr int L2 = S::lrs(1), U2 = 16 >> L2;
+    static constexpr int L3 = S::nstages > 2 ? S::lrs(2) : 0, U3 = L3 ? 16 >> L3 : 0;
+    float2 a[U2 * L2];
+    float2 b[U3 ? U3 * L3 : 1];
+    __device__ __forceinline__ StageRegs(const float2* __restrict__ tw, int t2, int t3)
+    {
+#pragma unroll
+        for (int u = 0; u < U2; ++u) {
+#pragma unroll
+            for (int i = 0; i < L2; ++i)
+                a[u * L2 + i] = tw_load<INV>(tw + (16 << L2 >> i), (t2 + u * T) & 15);
+        }
+#pragma unroll
+        for (int u = 0; u < U3; ++u) {
+#pragma unroll
+            for (int i = 0; i < L3; ++i)
+                b[u * L3 + i] = tw_load<INV>(tw + (256 << L3 >> i), (t3 + u * T) & 255);
+        }
+    }
+    template <int LEVEL, int U>
+    __device__ __forceinline__ float2 get(int) const
+    {
+        if constexpr (LEVEL <= (16 << L2)) return a[U * L2 + ilog2((16 << L2) / LEVEL)];
+        else return b[U * L3 + ilog2((256 << L3) / LEVEL)];
     }
 };
 
@@ -207,7 +224,7 @@ __device__ __forceinline__ void stage_compute(cpair (&v)[1 << LOG2R], int t, con
             float2 w[RS];
             static_for<0, LRS>([&](auto ic) {
                 constexpr int p = 1 << decltype(ic)::value;
-                w[p] = tab.template get<NS * RS / p>(k);
+                w[p] = tab.template get<NS * RS / p, u>(k);
             });
 #pragma unroll
             for (int j = 3; j < RS; ++j) {
