@@ -59,6 +59,52 @@ k_rows(const float2* __restrict__ in, float2* __restrict__ out, int log2n1, long
                           smem, tw, LB, [] { pdl_wait_then_launch(); });
 }
 
+// Passes 1 and 2 of the three-pass transform, one step of a chain of launches.
+// A panel -- gc neighbouring n3 of one transform, every n1 and n2 -- is closed
+// under both passes.  Step s runs pass 1 on panel s and pass 2 (in place) on
+// panel s - 1, tile by tile alternating, so the panels between the passes
+// (16-32 MB) are read back from L2: HBM sees both passes as one.  The pass-1
+// tiles depend on nothing in the chain, so they do not wait for the step before
+// (only step 0 waits, for the work ahead of the call); the pass-2 tiles do.  A
+// step lets the next one in once its own tiles have passed their waits, so a
+// step's start means that the step before the previous one is complete, and
+// the next step's pass-1 tiles fill this step's tail.
+template <int L1, int L2>
+struct Cols12 {
+    static constexpr int THREADS = 8 * (1 << ((L1 > L2 ? L1 : L2) - 4));
+    using P1 = PairCfg<L1, THREADS>;
+    using P2 = PairCfg<L2, THREADS>;
+    static_assert(P1::THREADS == THREADS && P2::THREADS == THREADS, "one tile a CTA");
+    static constexpr size_t SMEM = P1::SMEM > P2::SMEM ? P1::SMEM : P2::SMEM;
+};
+template <int L1, int L2, bool INV>
+__global__ void __launch_bounds__((Cols12<L1, L2>::THREADS), (65536 / (Cols12<L1, L2>::THREADS * 128)))
+k_cols12(const float2* __restrict__ in, float2* __restrict__ mid, int l3, int lgc, int s, int panels, long long in_dist,
+         const float2* __restrict__ tw)
+{
+    using P1 = typename Cols12<L1, L2>::P1;
+    using P2 = typename Cols12<L1, L2>::P2;
+    extern __shared__ __align__(128) cpair smem[];
+    const bool both = s > 0 && s < panels;
+    const int i = both ? blockIdx.x >> 1 : blockIdx.x;
+    const bool second = both ? blockIdx.x & 1 : s > 0;
+    const int panel = second ? s - 1 : s, lper = l3 - lgc;              // panels of one transform: 2^lper
+    const long long f = panel >> lper;
+    const int n3 = (panel & ((1 << lper) - 1)) << lgc;
+    if (!second) {
+        const int lt = lgc - ilog2(P1::C), n2 = i >> lt, c0 = n3 + ((i & ((1 << lt) - 1)) << ilog2(P1::C));
+        pair_cols<L1, INV, P1>(in + f * in_dist, mid + (f << (L1 + L2 + l3)), L2 + l3, ((n2 << l3) + c0) >> ilog2(P1::C),
+                               threadIdx.x, smem, tw, [s] {
+                                   if (s == 0) pdl_wait();
+                                   pdl_launch_dependents();
+                               });
+    } else {
+        const int lt = lgc - ilog2(P2::C), k1 = i >> lt, c0 = n3 + ((i & ((1 << lt) - 1)) << ilog2(P2::C));
+        float2* row = mid + (f << (L1 + L2 + l3)) + ((long long)k1 << (L2 + l3));
+        pair_cols<L2, INV, P2>(row, row, l3, c0 >> ilog2(P2::C), threadIdx.x, smem, tw, [] { pdl_wait_then_launch(); });
+    }
+}
+
 // Third pass of the three-pass transform (N = N1 N2 N3, sub-lengths 2^l1,
 // 2^l2, 2^LB): block (f, k2, tile) runs DFT_N3 along the C rows k1 of the
 // tile, row (k1, k2) of transform f at in[f N + k1 N2 N3 + k2 N3 ..], and
@@ -190,6 +236,43 @@ static cudaError_t launch_rows3(int l3, const float2* in, float2* out, long long
     }
 }
 
+// Bytes of a panel of the chained passes 1 and 2.
+constexpr int kPanelLog2 = 24;
+
+template <int L1, int L2, bool INV>
+static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long long count, long long in_dist,
+                                   const float2* tw, cudaStream_t s)
+{
+    using C = Cols12<L1, L2>;
+    int lgc = kPanelLog2 - 3 - L1 - L2;
+    if (lgc < 5) lgc = 5;
+    if (lgc > l3) lgc = l3;
+    const int panels = (int)(count << (l3 - lgc));
+    const unsigned tiles = 1u << (L1 + L2 + lgc - ilog2(C::THREADS * 32));
+    for (int st = 0; st <= panels; ++st) {
+        const unsigned blocks = st > 0 && st < panels ? 2 * tiles : tiles;
+        const cudaError_t e = launch_pdl(k_cols12<L1, L2, INV>, dim3(blocks), dim3(C::THREADS), C::SMEM, s, in, mid, l3, lgc,
+                                         st, panels, in_dist, tw);
+        if (e != cudaSuccess) return e;
+        count_launch();
+    }
+    return cudaSuccess;
+}
+
+template <bool INV>
+static cudaError_t launch_cols12(int l1, int l2, int l3, const float2* in, float2* mid, long long count, long long in_dist,
+                                 const float2* tw, cudaStream_t s)
+{
+    switch (l1 * 16 + l2) {
+    case 7 * 16 + 7: return launch_cols12_L<7, 7, INV>(in, mid, l3, count, in_dist, tw, s);
+    case 7 * 16 + 8: return launch_cols12_L<7, 8, INV>(in, mid, l3, count, in_dist, tw, s);
+    case 8 * 16 + 8: return launch_cols12_L<8, 8, INV>(in, mid, l3, count, in_dist, tw, s);
+    case 8 * 16 + 9: return launch_cols12_L<8, 9, INV>(in, mid, l3, count, in_dist, tw, s);
+    case 9 * 16 + 9: return launch_cols12_L<9, 9, INV>(in, mid, l3, count, in_dist, tw, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 // Three sub-lengths of at most 2^10 (each >= 2^7), as equal as possible.
 static bool plan3(int log2n, int* l1, int* l2, int* l3)
 {
@@ -226,15 +309,18 @@ static cudaError_t launch_three_pass(Kind kind, int log2n, const float2* in, flo
         const long long cnt = count - off < group ? count - off : group;
         const float2* src = in + off * in_dist;
         float2* dst = out + off * out_dist;
-        // pass 1: columns of length N1 over the M = N2 N3 columns -> tmp
-        cudaError_t e = kind == C2R       ? launch_cols_merge(l1, src, tmp, cnt, l2 + l3, in_dist, n, tw, s)
-                        : inverse         ? launch_cols<true>(l1, src, tmp, cnt, l2 + l3, in_dist, n, tw, s)
-                                          : launch_cols<false>(l1, src, tmp, cnt, l2 + l3, in_dist, n, tw, s);
-        // pass 2: in every row k1, columns of length N2 over the N3 columns, in place
-        if (e == cudaSuccess)
-            e = inverse ? launch_cols<true>(l2, tmp, tmp, cnt << l1, l3, M, M, tw, s)
-                        : launch_cols<false>(l2, tmp, tmp, cnt << l1, l3, M, M, tw, s);
-        count_launch(2);
+        cudaError_t e;
+        if (kind != C2R) {
+            e = inverse ? launch_cols12<true>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s)
+                        : launch_cols12<false>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s);
+        } else {
+            // pass 1: columns of length N1 over the M = N2 N3 columns -> tmp,
+            // with the merge (its tiles mirror across panels); pass 2: in every
+            // row k1, columns of length N2 over the N3 columns, in place
+            e = launch_cols_merge(l1, src, tmp, cnt, l2 + l3, in_dist, n, tw, s);
+            if (e == cudaSuccess) e = launch_cols<true>(l2, tmp, tmp, cnt << l1, l3, M, M, tw, s);
+            count_launch(2);
+        }
         // pass 3: rows of length N3, C consecutive k1 per tile -> out (real
         // forward: row pairs k, N1 N2 - k with the split)
         if (e == cudaSuccess)
@@ -470,6 +556,15 @@ cudaError_t launch_large_c2r(int log2n, const void* in, void* out, long long cou
     return cudaErrorInvalidValue;
 }
 
+template <int L1, int L2>
+static cudaError_t attr_cols12()
+{
+    const int smem = (int)Cols12<L1, L2>::SMEM;
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_cols12<L1, L2, false>, a, smem);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k_cols12<L1, L2, true>, a, smem) : e;
+}
+
 template <int L>
 static cudaError_t attr_pass()
 {
@@ -491,6 +586,11 @@ cudaError_t prepare_large()
     if (e == cudaSuccess) e = attr_pass<8>();
     if (e == cudaSuccess) e = attr_pass<9>();
     if (e == cudaSuccess) e = attr_pass<10>();
+    if (e == cudaSuccess) e = attr_cols12<7, 7>();
+    if (e == cudaSuccess) e = attr_cols12<7, 8>();
+    if (e == cudaSuccess) e = attr_cols12<8, 8>();
+    if (e == cudaSuccess) e = attr_cols12<8, 9>();
+    if (e == cudaSuccess) e = attr_cols12<9, 9>();
     return e;
 }
 
