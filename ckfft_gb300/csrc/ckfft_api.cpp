@@ -665,6 +665,8 @@ cudaError_t enqueue_strided(CkFftContext* c, const Work& w, const void* in, long
     }
     // consecutive transforms adjacent (interleaved channels, matrix columns)
     const bool cin = w.in_dist == 1 && is > 1, cout = w.out_dist == 1 && os > 1;
+    if (cin && cout && ckg::columns_apply(w.kind, w.log2n, in, out, is, os))
+        return ckg::launch_columns(w.kind, w.log2n, in, out, w.count, is, os, c->dtw, s);
     const bool complex_in_only = !is_real(w.kind) && cin && !cout && w.log2n >= 12;
     if (!complex_in_only && ckg::inter_applies(w.kind, w.log2n, cin, cout))
         return ckg::launch_inter(w.kind, w.log2n, in, out, w.count, ckg::Layout{is, w.in_dist, os, w.out_dist}, cin,

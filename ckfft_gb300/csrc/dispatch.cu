@@ -22,6 +22,7 @@ cudaError_t prepare_inter();
 cudaError_t prepare_l2pass();
 cudaError_t prepare_groups();
 cudaError_t prepare_flow();
+cudaError_t prepare_columns();
 cudaError_t prepare_shape_halfr();
 cudaError_t prepare_shape_doubler();
 cudaError_t prepare_shape_cta512();
@@ -249,6 +250,7 @@ cudaError_t prepare_device()
     if ((e = prepare_l2pass()) != cudaSuccess) return e;
     if ((e = prepare_groups()) != cudaSuccess) return e;
     if ((e = prepare_flow()) != cudaSuccess) return e;
+    if ((e = prepare_columns()) != cudaSuccess) return e;
     if ((e = prepare_shape_halfr()) != cudaSuccess) return e;
     if ((e = prepare_shape_doubler()) != cudaSuccess) return e;
     if ((e = prepare_shape_cta512()) != cudaSuccess) return e;

@@ -9,6 +9,9 @@
 // sector per element.  The transforms then run from the slots exactly as in
 // the batched kernels.
 //
+// Where both sides are distance 1, fft_columns.cu takes complex 2^8 .. 2^12 and
+// real n = 2^9 .. 2^13 (all but its smallest sizes where rows are unaligned).
+//
 // Covered: complex 2^6 .. 2^13 (either side or both interleaved), real
 // forward with interleaved reals, real inverse with interleaved reals, real
 // n = 2^7 .. 2^14.  G is at least 16 (rows of 128 bytes and more) up to

@@ -46,6 +46,12 @@ cudaError_t launch_strided(Kind kind, int log2n, const void* in, void* out, long
 bool inter_applies(Kind kind, int log2n, bool cin, bool cout);
 cudaError_t launch_inter(Kind kind, int log2n, const void* in, void* out, long long count, const Layout& lay,
                          bool cin, bool cout, const float2* tw, cudaStream_t stream);
+// Both sides distance 1 (element p of transform f at [p * stride + f]): two
+// columns a thread straight between memory and registers (fft_columns.cu).
+// Complex 2^8..2^12, real 2^9..2^13 (not the smallest where rows are unaligned).
+bool columns_apply(Kind kind, int log2n, const void* in, const void* out, long long in_stride, long long out_stride);
+cudaError_t launch_columns(Kind kind, int log2n, const void* in, void* out, long long count, long long in_stride,
+                           long long out_stride, const float2* tw, cudaStream_t stream);
 // `count` rows of `len` elements of `esize` bytes (4 or 8) between the
 // strided layout (stride, dist) and contiguous rows.
 cudaError_t launch_gather(const void* src, long long stride, long long dist, void* dst, long long count,
