@@ -33,7 +33,7 @@ using BPass = PairCfg<LS, 256, 8>;
 template <int LS>
 constexpr int kPassBlocks = 65536 / (BPass<LS>::THREADS * 128);
 
-template <int LA, bool INV>
+template <int LA, bool INV, bool MIRROR>
 __global__ void __launch_bounds__(BPass<LA>::THREADS, kPassBlocks<LA>)
 k_cols(const float2* __restrict__ in, float2* __restrict__ out, int log2n2, long long in_dist, long long out_dist,
        const float2* __restrict__ tw)
@@ -42,7 +42,7 @@ k_cols(const float2* __restrict__ in, float2* __restrict__ out, int log2n2, long
     extern __shared__ __align__(128) cpair smem[];
     const int log2tiles = log2n2 - ilog2(P::C);
     const long long f = blockIdx.x >> log2tiles;
-    pair_cols<LA, INV, P>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
+    pair_cols<LA, INV, MIRROR, P>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
                           smem, tw, [] { pdl_wait_then_launch(); });
 }
 
@@ -77,7 +77,7 @@ struct Cols12 {
     static_assert(P1::THREADS == THREADS && P2::THREADS == THREADS, "one tile a CTA");
     static constexpr size_t SMEM = P1::SMEM > P2::SMEM ? P1::SMEM : P2::SMEM;
 };
-template <int L1, int L2, bool INV>
+template <int L1, int L2, bool INV, bool MIRROR>
 __global__ void __launch_bounds__((Cols12<L1, L2>::THREADS), (65536 / (Cols12<L1, L2>::THREADS * 128)))
 k_cols12(const float2* __restrict__ in, float2* __restrict__ mid, int l3, int lgc, int s, int panels, long long in_dist,
          const float2* __restrict__ tw)
@@ -93,7 +93,7 @@ k_cols12(const float2* __restrict__ in, float2* __restrict__ mid, int l3, int lg
     const int n3 = (panel & ((1 << lper) - 1)) << lgc;
     if (!second) {
         const int lt = lgc - ilog2(P1::C), n2 = i >> lt, c0 = n3 + ((i & ((1 << lt) - 1)) << ilog2(P1::C));
-        pair_cols<L1, INV, P1>(in + f * in_dist, mid + (f << (L1 + L2 + l3)), L2 + l3, ((n2 << l3) + c0) >> ilog2(P1::C),
+        pair_cols<L1, INV, false, P1>(in + f * in_dist, mid + (f << (L1 + L2 + l3)), L2 + l3, ((n2 << l3) + c0) >> ilog2(P1::C),
                                threadIdx.x, smem, tw, [s] {
                                    if (s == 0) pdl_wait();
                                    pdl_launch_dependents();
@@ -101,7 +101,8 @@ k_cols12(const float2* __restrict__ in, float2* __restrict__ mid, int l3, int lg
     } else {
         const int lt = lgc - ilog2(P2::C), k1 = i >> lt, c0 = n3 + ((i & ((1 << lt) - 1)) << ilog2(P2::C));
         float2* row = mid + (f << (L1 + L2 + l3)) + ((long long)k1 << (L2 + l3));
-        pair_cols<L2, INV, P2>(row, row, l3, c0 >> ilog2(P2::C), threadIdx.x, smem, tw, [] { pdl_wait_then_launch(); });
+        pair_cols<L2, INV, MIRROR, P2>(row, row, l3, c0 >> ilog2(P2::C), threadIdx.x, smem, tw,
+                                       [] { pdl_wait_then_launch(); }, k1 == 0);
     }
 }
 
@@ -126,57 +127,60 @@ k_rows3(const float2* __restrict__ in, float2* __restrict__ out, int l1, int l2,
                           l2 + LB, [] { pdl_wait_then_launch(); });
 }
 
-// The split and merge passes run one value a thread (fft_passes.cuh), 512
-// threads and 64 registers: two values a thread measured slower there, more so
-// with other streams' kernels (real 2^18 x 127 forward 111 -> 114 us, a pair on
-// three streams 207 -> 218; 2^21 x 16 inverse 155 -> 163): the mirrored halves
-// leave stores of 8 bytes and loads of single bins, which want warps in flight.
+// The split and merge passes: a pair is a row (column) and its mirror, and the
+// split or merge happens inside the pair's registers.  With one value a thread
+// (512 threads, 64 registers) the mirror had to be found through shared
+// memory, and shared memory was the bound (77-79 % of its rate, HBM at 40 %):
+// five accesses a value for the merge and six for the split, two and four now.
+// 8-byte stores (loads) of up to 16 neighbours either way; 256 threads against
+// 512 (real 2^20 x 32, a forward and an inverse: 232 against 255 us), 16 pairs
+// against 8 (2^22 x 8: 255 against 271).  Before and after, us: 2^18 x 127 228
+// -> 203, 2^20 x 32 287 -> 234, 2^22 x 8 307 -> 256, 2^24 x 2 316 -> 259, 2^22
+// alone 50 -> 39.
 template <int LS>
-using SPass = PassCfg<LS, 512>;
+using SPass = PairCfg<LS, 256, 16>;
 template <int LS>
-constexpr int kSplitBlocks = 65536 / (SPass<LS>::THREADS * 64);
+constexpr int kSplitBlocks = 65536 / (SPass<LS>::THREADS * 128);
 
 // Row pass of a real forward transform with the split fused: block
-// (f, tile) writes the M+1 output bins of its row pairs (pass_rows_split).
+// (f, tile) writes the M+1 output bins of its row pairs (pair_rows_split).
 template <int LB>
 __global__ void __launch_bounds__(SPass<LB>::THREADS, kSplitBlocks<LB>)
 k_rows_split(const float2* __restrict__ in, float2* __restrict__ out, int log2n1, int log2k1, long long in_dist,
              long long out_dist, const float2* __restrict__ tw)
 {
     using P = SPass<LB>;
-    extern __shared__ __align__(128) float2 smem1[];
-    pdl_wait_then_launch();
+    extern __shared__ __align__(128) cpair smem[];
     const int log2tiles = log2n1 - ilog2(P::C);
     const long long f = blockIdx.x >> log2tiles;
-    pass_rows_split<LB, 512>(in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x & ((1 << log2tiles) - 1),
-                             threadIdx.x, smem1, tw, log2k1);
+    pair_rows_split<LB, P>(in + f * in_dist, out + f * out_dist, log2n1, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
+                           smem, tw, log2k1, [] { pdl_wait_then_launch(); });
 }
 
 // Column pass of a real inverse transform with the merge fused: block
-// (f, tile) reads the M+1 bins of its column pairs (pass_cols_merge).
+// (f, tile) reads the M+1 bins of its column pairs (pair_cols_merge).
 template <int LA>
 __global__ void __launch_bounds__(SPass<LA>::THREADS, kSplitBlocks<LA>)
 k_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2, long long in_dist,
              long long out_dist, const float2* __restrict__ tw)
 {
     using P = SPass<LA>;
-    extern __shared__ __align__(128) float2 smem1[];
-    pdl_wait_then_launch();
+    extern __shared__ __align__(128) cpair smem[];
     const int log2tiles = log2n2 - ilog2(P::C);
     const long long f = blockIdx.x >> log2tiles;
-    pass_cols_merge<LA, 512>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1),
-                             threadIdx.x, smem1, tw);
+    pair_cols_merge<LA, P>(in + f * in_dist, out + f * out_dist, log2n2, blockIdx.x & ((1 << log2tiles) - 1), threadIdx.x,
+                           smem, tw, [] { pdl_wait_then_launch(); });
 }
 
 // ---------------------------------------------------------------- launch
 
-template <int LA, bool INV>
+template <int LA, bool INV, bool MIRROR>
 static cudaError_t launch_cols_L(const float2* in, float2* out, long long count, int log2n2,
                                  long long in_dist, long long out_dist, const float2* tw, cudaStream_t s)
 {
     using P = BPass<LA>;
     const long long blocks = count * ((1ll << log2n2) / P::C);
-    return launch_pdl(k_cols<LA, INV>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n2, in_dist,
+    return launch_pdl(k_cols<LA, INV, MIRROR>, dim3((unsigned)blocks), dim3(P::THREADS), P::SMEM, s, in, out, log2n2, in_dist,
                       out_dist, tw);
 }
 
@@ -190,27 +194,31 @@ static cudaError_t launch_rows_L(const float2* in, float2* out, long long count,
                       out_dist, tw);
 }
 
-#define CKG_SUB_SWITCH(L, FN, ...)                                                                 \
-    switch (L) {                                                                                   \
-    case 7: return FN<7, INV>(__VA_ARGS__);                                                        \
-    case 8: return FN<8, INV>(__VA_ARGS__);                                                        \
-    case 9: return FN<9, INV>(__VA_ARGS__);                                                        \
-    case 10: return FN<10, INV>(__VA_ARGS__);                                                      \
-    default: return cudaErrorInvalidValue;                                                         \
-    }
-
-template <bool INV>
+// MIRROR: of a real forward transform (pair_rows_split reads the result).
+template <bool INV, bool MIRROR = false>
 static cudaError_t launch_cols(int la, const float2* in, float2* out, long long count, int log2n2,
                                long long in_dist, long long out_dist, const float2* tw, cudaStream_t s)
 {
-    CKG_SUB_SWITCH(la, launch_cols_L, in, out, count, log2n2, in_dist, out_dist, tw, s)
+    switch (la) {
+    case 7: return launch_cols_L<7, INV, MIRROR>(in, out, count, log2n2, in_dist, out_dist, tw, s);
+    case 8: return launch_cols_L<8, INV, MIRROR>(in, out, count, log2n2, in_dist, out_dist, tw, s);
+    case 9: return launch_cols_L<9, INV, MIRROR>(in, out, count, log2n2, in_dist, out_dist, tw, s);
+    case 10: return launch_cols_L<10, INV, MIRROR>(in, out, count, log2n2, in_dist, out_dist, tw, s);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 template <bool INV>
 static cudaError_t launch_rows(int lb, const float2* in, float2* out, long long count, int log2n1,
                                long long in_dist, long long out_dist, const float2* tw, cudaStream_t s)
 {
-    CKG_SUB_SWITCH(lb, launch_rows_L, in, out, count, log2n1, in_dist, out_dist, tw, s)
+    switch (lb) {
+    case 7: return launch_rows_L<7, INV>(in, out, count, log2n1, in_dist, out_dist, tw, s);
+    case 8: return launch_rows_L<8, INV>(in, out, count, log2n1, in_dist, out_dist, tw, s);
+    case 9: return launch_rows_L<9, INV>(in, out, count, log2n1, in_dist, out_dist, tw, s);
+    case 10: return launch_rows_L<10, INV>(in, out, count, log2n1, in_dist, out_dist, tw, s);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 template <int LB, bool INV>
@@ -239,7 +247,7 @@ static cudaError_t launch_rows3(int l3, const float2* in, float2* out, long long
 // Bytes of a panel of the chained passes 1 and 2.
 constexpr int kPanelLog2 = 24;
 
-template <int L1, int L2, bool INV>
+template <int L1, int L2, bool INV, bool MIRROR>
 static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long long count, long long in_dist,
                                    const float2* tw, cudaStream_t s)
 {
@@ -251,7 +259,7 @@ static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long l
     const unsigned tiles = 1u << (L1 + L2 + lgc - ilog2(C::THREADS * 32));
     for (int st = 0; st <= panels; ++st) {
         const unsigned blocks = st > 0 && st < panels ? 2 * tiles : tiles;
-        const cudaError_t e = launch_pdl(k_cols12<L1, L2, INV>, dim3(blocks), dim3(C::THREADS), C::SMEM, s, in, mid, l3, lgc,
+        const cudaError_t e = launch_pdl(k_cols12<L1, L2, INV, MIRROR>, dim3(blocks), dim3(C::THREADS), C::SMEM, s, in, mid, l3, lgc,
                                          st, panels, in_dist, tw);
         if (e != cudaSuccess) return e;
         count_launch();
@@ -259,16 +267,16 @@ static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long l
     return cudaSuccess;
 }
 
-template <bool INV>
+template <bool INV, bool MIRROR>
 static cudaError_t launch_cols12(int l1, int l2, int l3, const float2* in, float2* mid, long long count, long long in_dist,
                                  const float2* tw, cudaStream_t s)
 {
     switch (l1 * 16 + l2) {
-    case 7 * 16 + 7: return launch_cols12_L<7, 7, INV>(in, mid, l3, count, in_dist, tw, s);
-    case 7 * 16 + 8: return launch_cols12_L<7, 8, INV>(in, mid, l3, count, in_dist, tw, s);
-    case 8 * 16 + 8: return launch_cols12_L<8, 8, INV>(in, mid, l3, count, in_dist, tw, s);
-    case 8 * 16 + 9: return launch_cols12_L<8, 9, INV>(in, mid, l3, count, in_dist, tw, s);
-    case 9 * 16 + 9: return launch_cols12_L<9, 9, INV>(in, mid, l3, count, in_dist, tw, s);
+    case 7 * 16 + 7: return launch_cols12_L<7, 7, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+    case 7 * 16 + 8: return launch_cols12_L<7, 8, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+    case 8 * 16 + 8: return launch_cols12_L<8, 8, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+    case 8 * 16 + 9: return launch_cols12_L<8, 9, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+    case 9 * 16 + 9: return launch_cols12_L<9, 9, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -311,8 +319,9 @@ static cudaError_t launch_three_pass(Kind kind, int log2n, const float2* in, flo
         float2* dst = out + off * out_dist;
         cudaError_t e;
         if (kind != C2R) {
-            e = inverse ? launch_cols12<true>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s)
-                        : launch_cols12<false>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s);
+            e = inverse       ? launch_cols12<true, false>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s)
+                : kind == R2C ? launch_cols12<false, true>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s)
+                              : launch_cols12<false, false>(l1, l2, l3, src, tmp, cnt, in_dist, tw, s);
         } else {
             // pass 1: columns of length N1 over the M = N2 N3 columns -> tmp,
             // with the merge (its tiles mirror across panels); pass 2: in every
@@ -442,7 +451,7 @@ static cudaError_t launch_r2c_rows_split(int lm, const float2* in, float2* out, 
     if (group < 1) return cudaErrorInvalidValue;
     for (long long off = 0; off < count; off += group) {
         const long long cnt = count - off < group ? count - off : group;
-        cudaError_t e = launch_cols<false>(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
+        cudaError_t e = launch_cols<false, true>(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
         if (e == cudaSuccess)
             e = launch_rows_split(p.log2n2, tmp, out + off * out_dist, cnt, p.log2n1, p.log2n1, M, out_dist, tw, s);
         if (e != cudaSuccess) return e;
@@ -561,8 +570,9 @@ static cudaError_t attr_cols12()
 {
     const int smem = (int)Cols12<L1, L2>::SMEM;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(k_cols12<L1, L2, false>, a, smem);
-    return e == cudaSuccess ? cudaFuncSetAttribute(k_cols12<L1, L2, true>, a, smem) : e;
+    cudaError_t e = cudaFuncSetAttribute(k_cols12<L1, L2, false, false>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols12<L1, L2, false, true>, a, smem);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k_cols12<L1, L2, true, false>, a, smem) : e;
 }
 
 template <int L>
@@ -574,8 +584,9 @@ static cudaError_t attr_pass()
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows3<L, true>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows_split<L>, a, (int)SPass<L>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols_merge<L>, a, (int)SPass<L>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, false>, a, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, true>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, false, false>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, false, true>, a, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols<L, true, false>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows<L, false>, a, smem);
     return e == cudaSuccess ? cudaFuncSetAttribute(k_rows<L, true>, a, smem) : e;
 }

@@ -80,6 +80,7 @@ __device__ __forceinline__ cpair cadd(cpair a, cpair b) { return {add2(a.x, b.x)
 __device__ __forceinline__ cpair csub(cpair a, cpair b) { return {sub2(a.x, b.x), sub2(a.y, b.y)}; }
 __device__ __forceinline__ cpair cadd_i(cpair a, cpair b) { return {sub2(a.x, b.y), add2(a.y, b.x)}; }
 __device__ __forceinline__ cpair csub_i(cpair a, cpair b) { return {add2(a.x, b.y), sub2(a.y, b.x)}; }
+__device__ __forceinline__ cpair conj2(cpair a) { return {a.x, neg2(a.y)}; }
 // lane-wise product, and the product with one value for both lanes
 __device__ __forceinline__ cpair cmul(cpair a, cpair w)
 {
