@@ -1,7 +1,8 @@
-"""Real transforms of several passes (n >= 2^18): the column pass that stores
+"""Real transforms of several passes (n >= 2^16): the column pass that stores
 mirrored rows conjugated, the row pass with the split in its registers and the
 column pass with the merge in its registers.  Every sub-length (2^7 .. 2^10),
-the two- and the three-pass plans, and the rows and columns that mirror
+the cluster kernel with
+eight and with four blocks a transform, the two- and the three-pass plans, and the rows and columns that mirror
 themselves (bins 0, M/2, M and the middle rows): every output against FP64.
 
 Tolerance: each of the log2 n levels rounds a handful of times at 2^-24 of a
@@ -22,7 +23,7 @@ def check(got, want, log2n):
     assert err.max() <= tol, (int(err.argmax()), float(err.max()), tol)
 
 
-@pytest.mark.parametrize("log2n,count", [(18, 3), (19, 2), (20, 2), (21, 1), (22, 2), (23, 1), (24, 1), (25, 1)])
+@pytest.mark.parametrize("log2n,count", [(16, 2), (16, 385), (17, 3), (18, 3), (19, 2), (20, 2), (21, 1), (22, 2), (23, 1), (24, 1), (25, 1)])
 def test_forward_and_inverse(torch_cuda, ctx_cache, log2n, count):
     torch, n = torch_cuda, 1 << log2n
     rng = np.random.default_rng(log2n)
