@@ -398,6 +398,32 @@ __device__ __forceinline__ void stage_exchange(float2 (&v)[1 << LOG2R], int t, c
     xsync<WARP, BAR_ID, BAR_N>();
 }
 
+// The exchange before a last stage of radix 2, by the 32 threads of a warp that
+// hold a whole transform (2^9 points, 16 values a thread).  That stage pairs
+// position p with p + N/2, which lane t + 16 holds where lane t holds p: each
+// lane sends half its values across and no value goes through shared memory
+// (a shuffle moves 4 bytes a lane in one access, the two-way exchange 16).
+// Positions as after stage_exchange: v[m] = t + m T.
+template <int LOG2N, int LOG2R>
+constexpr bool kShuffleLast = LOG2N == 9 && LOG2R == 4;
+template <int R>
+__device__ __forceinline__ void exchange_shuffle(float2 (&v)[R], int t)
+{
+    const bool hi = t & 16;
+    float2 r[R];
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i) {
+        // output j of this lane's butterfly sits at (t & 16) * 16 + (t & 15) + 16 j:
+        // the low lane takes the even j of both halves, the high lane the odd
+        const float2 send = hi ? v[2 * i] : v[2 * i + 1], keep = hi ? v[2 * i + 1] : v[2 * i];
+        const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, send.x, 16), __shfl_xor_sync(0xffffffffu, send.y, 16));
+        r[i] = hi ? got : keep;
+        r[i + R / 2] = hi ? keep : got;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = r[i];
+}
+
 // Full transform of one length-2^LOG2N sequence held as v[m] = x[t + m*T].
 // On return v[m] = X[t + m*T].  The view must not be in use by other code
 // between the call's barriers.
@@ -413,7 +439,8 @@ __device__ __forceinline__ void stockham(float2 (&v)[1 << LOG2R], int t, const f
             constexpr int s = decltype(sc)::value;
             constexpr int lrs = S::lrs(s), lns = S::lns(s);
             stage_compute<LOG2N, LOG2R, lrs, lns, INV>(v, t, tw);
-            if constexpr (s + 1 < S::nstages)
+            if constexpr (WARP && kShuffleLast<LOG2N, LOG2R> && s + 2 == S::nstages) exchange_shuffle(v, t);
+            else if constexpr (s + 1 < S::nstages)
                 stage_exchange<LOG2N, LOG2R, lrs, lns, WARP, BAR_ID, BAR_N>(v, t, view);
         });
     }

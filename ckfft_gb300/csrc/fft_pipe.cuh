@@ -99,10 +99,14 @@ k_pipe(const float2* __restrict__ in, float2* __restrict__ out, long long ngroup
         const long long f = grp * C::TPB + g;
         if constexpr (KIND == R2C) {
             constexpr int M = N;
+            if constexpr (kMirrorShuffle<C>) {
+                split_store_warp<C, M>(v, RowOut{out + f * out_dist}, true, t, tw + 2 * M);
+            } else {
 #pragma unroll
-            for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, v[m]);
-            xsync<C::WARP>();
-            split_store<C, M>(view, RowOut{out + f * out_dist}, t, tw + 2 * M);
+                for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, v[m]);
+                xsync<C::WARP>();
+                split_store<C, M>(view, RowOut{out + f * out_dist}, t, tw + 2 * M);
+            }
         } else {
             float2* dst = out + f * out_dist + t;
 #pragma unroll

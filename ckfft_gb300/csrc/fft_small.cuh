@@ -133,6 +133,48 @@ __device__ __forceinline__ void split_store(const View& view, const Dst& dst, in
     }
 }
 
+// A frame held by part of a warp (16 or 32 threads, v[m] = position t + m T):
+// position M - (t + m T) is value R - 1 - m of lane T - t (lane 0 mirrors
+// itself: value R - m).  mirror_of(v, m) fetches it, for m >= 1 in lane 0;
+// called by all lanes.
+template <class C>
+constexpr bool kMirrorShuffle = C::WARP && (C::T == 16 || C::T == 32) && C::R >= 4;
+template <class C, int M_>
+__device__ __forceinline__ float2 mirror_of(const float2 (&v)[C::R], int t)
+{
+    const float2 a = v[C::R - 1 - M_];
+    float2 b = make_float2(__shfl_sync(0xffffffffu, a.x, (C::T - t) & (C::T - 1), C::T),
+                           __shfl_sync(0xffffffffu, a.y, (C::T - t) & (C::T - 1), C::T));
+    if (t == 0) b = v[M_ == 0 ? 0 : C::R - M_];
+    return b;
+}
+
+// split_store with the spectrum in the frame's registers (kMirrorShuffle): half
+// the values cross lanes, none go through shared memory.
+template <class C, int M, class Dst>
+__device__ __forceinline__ void split_store_warp(const float2 (&v)[C::R], const Dst& dst, bool live, int t,
+                                                 const float2* __restrict__ twn)
+{
+    const float2 w0 = __ldg(twn + t);
+    static_for<0, C::R / 2>([&](auto mc) {
+        constexpr int m = decltype(mc)::value;
+        const int k = t + m * C::T;
+        const float2 z0 = v[m], z1 = mirror_of<C, m>(v, t);
+        const float2 w = split_twiddle<C::R, m, false>(w0, twn, k);
+        const float sx = z0.x + z1.x, sy = z0.y - z1.y;
+        const float dx = z0.x - z1.x, dy = z0.y + z1.y;
+        const float px = fmaf(w.x, dx, -w.y * dy), py = fmaf(w.x, dy, w.y * dx);
+        if (live) {
+            dst.st(k, make_float2(sx + py, sy - px));
+            dst.st(M - k, make_float2(sx - py, -(sy + px)));
+        }
+    });
+    if (live && t == 0) {
+        const float2 z = v[C::R / 2];                   // X[M/2] = 2 conj Z[M/2]
+        dst.st(M / 2, make_float2(z.x + z.x, -(z.y + z.y)));
+    }
+}
+
 // ------------------------------------------------------- one-frame bodies
 // The T threads t = 0..T-1 of a group transform one frame between device
 // pointers; `live == false` keeps the group in step (barriers) without
@@ -180,11 +222,15 @@ __device__ __forceinline__ void frame_r2c_at(const Src& src, const Dst& dst, boo
         for (int m = 0; m < C::R; ++m) v[m] = make_float2(0.f, 0.f);
     }
     stockham<LM, C::LOG2R, false, C::WARP>(v, t, tw, view);
-    // natural-order half-size spectrum Z to shared memory, then split
+    if constexpr (kMirrorShuffle<C>) {
+        split_store_warp<C, M>(v, dst, live, t, tw + 2 * M);
+    } else {
+        // natural-order half-size spectrum Z to shared memory, then split
 #pragma unroll
-    for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, v[m]);
-    xsync<C::WARP>();
-    if (live) split_store<C, M>(view, dst, t, tw + 2 * M);
+        for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, v[m]);
+        xsync<C::WARP>();
+        if (live) split_store<C, M>(view, dst, t, tw + 2 * M);
+    }
 }
 
 template <int LM>
