@@ -94,40 +94,6 @@ k_stft(const float* __restrict__ signal, long long hop, const float* __restrict_
                      f < count, t, PaddedView{smem + g * C::SLOT}, tw);
 }
 
-// The merge of a frame whose bins are products: each bin is fetched and
-// multiplied once and its mirror passed on -- across lanes where the frame is
-// in one warp, else through the frame's shared memory -- where c2r_load would
-// fetch and form it twice (the second fetch of the bins missed L1: 457 MB of L2
-// reads for 246 MB of traffic at n = 1024).
-template <int LM, class Src>
-__device__ __forceinline__ void product_c2r_load(const Src& src, bool live, int t, const PaddedView& view,
-                                                 const float2* __restrict__ tw, float2 (&v)[SmallCfg<LM>::R])
-{
-    using C = SmallCfg<LM>;
-    constexpr int M = 1 << LM;
-    const float2* twn = tw + 2 * M;
-    float2 a[C::R], last = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int m = 0; m < C::R; ++m) a[m] = live ? src.ld(t + m * C::T) : make_float2(0.f, 0.f);
-    if (live && t == 0) last = src.ld(M);
-    const float2 w0 = __ldg(twn + t);
-    if constexpr (!kMirrorShuffle<C>) {
-#pragma unroll
-        for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, a[m]);
-        xsync<C::WARP>();
-    }
-    static_for<0, C::R>([&](auto mc) {
-        constexpr int m = decltype(mc)::value;
-        const int p = t + m * C::T;
-        float2 b;
-        if constexpr (kMirrorShuffle<C>) b = mirror_of<C, m>(a, t);
-        else b = view.ld((M - p) & (M - 1));
-        if (m == 0 && t == 0) b = last;
-        v[m] = real_merge(a[m], b, split_twiddle<C::R, m, false>(w0, twn, p));
-    });
-    if constexpr (!kMirrorShuffle<C>) xsync<C::WARP>();
-}
-
 template <int LM, bool FILT>
 __global__ void __launch_bounds__(SmallCfg<LM>::THREADS, SmallCfg<LM>::MINB)
 k_filter_c2r(const float2* __restrict__ spectra, const float2* __restrict__ filter, float scale,
@@ -139,15 +105,8 @@ k_filter_c2r(const float2* __restrict__ spectra, const float2* __restrict__ filt
     const int g = threadIdx.x / C::T, t = threadIdx.x % C::T;
     const long long f = (long long)blockIdx.x * C::TPB + g;
     const long long fc = f < count ? f : 0;
-    const PaddedView view{smem + g * C::SLOT};
-    float2 v[C::R];
-    product_c2r_load<LM>(FilterIn<FILT>{spectra + fc * (M + 1), filter, scale}, f < count, t, view, tw, v);
-    stockham<LM, C::LOG2R, true, C::WARP>(v, t, tw, view);
-    if (f < count) {
-        const RowOut dst{out + fc * M};
-#pragma unroll
-        for (int m = 0; m < C::R; ++m) dst.st(t + m * C::T, v[m]);
-    }
+    frame_c2r_at<LM>(FilterIn<FILT>{spectra + fc * (M + 1), filter, scale}, RowOut{out + fc * M}, f < count, t,
+                     PaddedView{smem + g * C::SLOT}, tw);
 }
 
 // Row passes of the generic route.

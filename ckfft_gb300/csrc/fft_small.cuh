@@ -268,12 +268,53 @@ __device__ __forceinline__ void c2r_load(const Src& src, bool live, int t, const
     }
 }
 
+// The same with each bin fetched once and its mirror passed on, across lanes
+// where the frame is in one warp (mirror_of), else through the frame's shared
+// memory.  Fetched twice, the second fetch is meant to hit L1 and often does
+// not: 457 MB of L2 reads for 246 MB of traffic in the filter kernel at n =
+// 1024, whose bins are products, formed twice as well.  Measured, batches of
+// 2^26 reals, us, fetched twice / once: n = 2^9 86.5 / 78.4, 2^10 91.5 / 83.2 (the
+// pipelined kernel, which reads pairs from its landing zone, 87.9), 2^11 97.5 /
+// 87.8 (92.6), 2^12 98.9 / 90.4 (94.5), 2^13 105.3 / 99.9.  Frames of fewer than 16
+// threads, which share lines among themselves, stay with two fetches (2^7 85.8 /
+// 98.7), and so does 2^15, where 32 values a thread leave no room (160 / 171).
+template <class C, int LM>
+constexpr bool kLoadOnce = C::T >= 16 && LM <= 13;
+template <int LM, class Src, class C = SmallCfg<LM>>
+__device__ __forceinline__ void c2r_load_once(const Src& src, bool live, int t, const PaddedView& view,
+                                                 const float2* __restrict__ tw, float2 (&v)[C::R])
+{
+    constexpr int M = 1 << LM;
+    const float2* twn = tw + 2 * M;
+    float2 a[C::R], last = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int m = 0; m < C::R; ++m) a[m] = live ? src.ld(t + m * C::T) : make_float2(0.f, 0.f);
+    if (live && t == 0) last = src.ld(M);
+    const float2 w0 = __ldg(twn + t);
+    if constexpr (!kMirrorShuffle<C>) {
+#pragma unroll
+        for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, a[m]);
+        xsync<C::WARP>();
+    }
+    static_for<0, C::R>([&](auto mc) {
+        constexpr int m = decltype(mc)::value;
+        const int p = t + m * C::T;
+        float2 b;
+        if constexpr (kMirrorShuffle<C>) b = mirror_of<C, m>(a, t);
+        else b = view.ld((M - p) & (M - 1));
+        if (m == 0 && t == 0) b = last;
+        v[m] = real_merge(a[m], b, split_twiddle<C::R, m, false>(w0, twn, p));
+    });
+    if constexpr (!kMirrorShuffle<C>) xsync<C::WARP>();
+}
+
 template <int LM, class Src, class Dst, class C = SmallCfg<LM>>
 __device__ __forceinline__ void frame_c2r_at(const Src& src, const Dst& dst, bool live, int t,
                                              const PaddedView& view, const float2* __restrict__ tw)
 {
     float2 v[C::R];
-    c2r_load<LM, Src, C>(src, live, t, tw, v);
+    if constexpr (kLoadOnce<C, LM>) c2r_load_once<LM, Src, C>(src, live, t, view, tw, v);
+    else c2r_load<LM, Src, C>(src, live, t, tw, v);
     stockham<LM, C::LOG2R, true, C::WARP>(v, t, tw, view);
     if (live) {
 #pragma unroll

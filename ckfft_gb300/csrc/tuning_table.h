@@ -1,5 +1,6 @@
 // tuning_table.h -- generated by ckfft_gb300/autotune.py; do not edit by hand.
-// Measured on NVIDIA GB300, 2026-12-04.
+// Measured on NVIDIA GB300, 2026-12-04; rinv 7 and 9 .. 11 again on 2026-12-05,
+// when the plain kernels had come to fetch each bin once.
 // kTunedLog2R[L]: values per thread (log2) of every single-CTA kernel family
 // (batched, pipelined, strided, fused, grouped, job kernel) for complex
 // (half-)length 2^L, so that all of them compute a size with the same radices.
@@ -15,6 +16,6 @@ constexpr signed char kTunedVariant[4][15] = {
     {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 7, 7, 0, 8, 8},   // cfwd
     {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 7, 7, 0, 0, 8},   // cinv
     {0, 0, 0, 0, 0, 0, 0, 7, 0, 7, 7, 7, 0, 0, 8},   // rfwd
-    {0, 0, 0, 0, 0, 0, 0, 0, 0, 2, 2, 2, 0, 8, 8},   // rinv
+    {0, 0, 0, 0, 0, 0, 0, 7, 0, 7, 7, 7, 0, 8, 8},   // rinv
 };
 }  // namespace ckg
