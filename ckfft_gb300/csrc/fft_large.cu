@@ -172,7 +172,98 @@ k_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2
                            smem, tw, [] { pdl_wait_then_launch(); });
 }
 
+// Both passes of a large batch of real transforms, one step of a chain of
+// launches as in k_cols12: a panel is `per` whole transforms (16 MB of
+// intermediates); step s runs the column pass on panel s, then the row pass on
+// panel s - 1, so the intermediates are read back from L2 and HBM sees the input
+// and the output once.  The column tiles come first: they need no wait, fill
+// the tail of the step before, and by the time the row tiles' turn comes that
+// step is complete (alternating tiles hold half the SMs in their waits: real
+// 2^18 x 127, a forward and an inverse, 226 us on one stream against 199).  Panels
+// of 32 MB measured 202 us on one stream and 192 on three, of 16 MB 199 and 175,
+// two launches over everything 206 and 192.  2^20 x 32: 237 / 219 us on one / three
+// streams in two launches, 220 / 197 here; 2^21 x 50 784 / 749 and 724 / 688.
+template <int LA, int LB>
+struct RealChain {
+    static constexpr int THREADS = 256;
+    using PA = PairCfg<LA, THREADS, 16>;
+    using PB = PairCfg<LB, THREADS, 16>;
+    static_assert(PA::THREADS == THREADS && PB::THREADS == THREADS, "one tile a CTA");
+    static constexpr int LOG2TILES = LA + LB - ilog2(32 * THREADS);      // tiles of one transform and pass
+    static constexpr size_t SMEM = PA::SMEM > PB::SMEM ? PA::SMEM : PB::SMEM;
+};
+template <int LA, int LB, bool INV>
+__global__ void __launch_bounds__(256, 2)
+k_real_chain(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict__ mid, int per, int s, int cols,
+             long long in_dist, long long out_dist, const float2* __restrict__ tw)
+{
+    using C = RealChain<LA, LB>;
+    extern __shared__ __align__(128) cpair smem[];
+    const bool second = (int)blockIdx.x >= cols;
+    const int i = second ? blockIdx.x - cols : blockIdx.x;
+    const int tile = i & ((1 << C::LOG2TILES) - 1);
+    const long long f = (long long)(second ? s - 1 : s) * per + (i >> C::LOG2TILES);
+    float2* m = mid + (f << (LA + LB));
+    if (!second) {
+        auto wait = [s] {
+            if (s == 0) pdl_wait();
+            pdl_launch_dependents();
+        };
+        if constexpr (INV) pair_cols_merge<LA, typename C::PA>(in + f * in_dist, m, LB, tile, threadIdx.x, smem, tw, wait);
+        else pair_cols<LA, false, true, typename C::PA>(in + f * in_dist, m, LB, tile, threadIdx.x, smem, tw, wait);
+    } else {
+        auto wait = [] { pdl_wait_then_launch(); };
+        if constexpr (INV) pair_rows<LB, true, typename C::PB>(m, out + f * out_dist, LA, tile, threadIdx.x, smem, tw, LB, wait);
+        else pair_rows_split<LB, typename C::PB>(m, out + f * out_dist, LA, tile, threadIdx.x, smem, tw, LA, wait);
+    }
+}
+
 // ---------------------------------------------------------------- launch
+
+// Bytes of a panel of the chained passes, and the values from which a batch of
+// real transforms is chained.
+constexpr int kPanelLog2 = 24;
+constexpr long long kChainMinPoints = 1ll << 22;
+
+template <int LA, int LB, bool INV>
+static cudaError_t launch_real_chain_L(const float2* in, float2* out, float2* mid, long long count, long long in_dist,
+                                       long long out_dist, const float2* tw, cudaStream_t s)
+{
+    using C = RealChain<LA, LB>;
+    constexpr long long per = 1ll << (kPanelLog2 - 3 - LA - LB);
+    const int panels = (int)((count + per - 1) / per);
+    auto tiles = [&](int p) { return p < 0 || p >= panels ? 0 : (int)((count - p * per < per ? count - p * per : per) << C::LOG2TILES); };
+    for (int st = 0; st <= panels; ++st) {
+        const int a = tiles(st), b = tiles(st - 1);
+        const cudaError_t e = launch_pdl(k_real_chain<LA, LB, INV>, dim3((unsigned)(a + b)), dim3(C::THREADS), C::SMEM, s, in,
+                                         out, mid, (int)per, st, a, in_dist, out_dist, tw);
+        if (e != cudaSuccess) return e;
+        count_launch();
+    }
+    return cudaSuccess;
+}
+
+// Half lengths 2^lm; in_dist / out_dist in float2.  *done: the batch ran here:
+// from 32 MB of intermediates on, two panels (2^18 x 32: 59 against 60 us; less of
+// it stays in L2 between two launches anyway), and where input and output do not
+// overlap (two launches read all inputs before the first output).
+template <bool INV>
+static cudaError_t launch_real_chain(int lm, const float2* in, float2* out, float2* mid, long long count, long long in_dist,
+                                     long long out_dist, const float2* tw, cudaStream_t s, bool* done)
+{
+    const long long n = 1ll << lm;
+    const char *i0 = (const char*)in, *i1 = (const char*)(in + (count - 1) * in_dist + n + 1);
+    const char *o0 = (const char*)out, *o1 = (const char*)(out + (count - 1) * out_dist + n + 1);
+    *done = (count << lm) >= kChainMinPoints && (i1 <= o0 || o1 <= i0);
+    if (!*done) return cudaSuccess;
+    switch (lm) {
+    case 17: return launch_real_chain_L<8, 9, INV>(in, out, mid, count, in_dist, out_dist, tw, s);
+    case 18: return launch_real_chain_L<9, 9, INV>(in, out, mid, count, in_dist, out_dist, tw, s);
+    case 19: return launch_real_chain_L<9, 10, INV>(in, out, mid, count, in_dist, out_dist, tw, s);
+    case 20: return launch_real_chain_L<10, 10, INV>(in, out, mid, count, in_dist, out_dist, tw, s);
+    default: *done = false; return cudaSuccess;
+    }
+}
 
 template <int LA, bool INV, bool MIRROR>
 static cudaError_t launch_cols_L(const float2* in, float2* out, long long count, int log2n2,
@@ -243,9 +334,6 @@ static cudaError_t launch_rows3(int l3, const float2* in, float2* out, long long
     default: return cudaErrorInvalidValue;
     }
 }
-
-// Bytes of a panel of the chained passes 1 and 2.
-constexpr int kPanelLog2 = 24;
 
 template <int L1, int L2, bool INV, bool MIRROR>
 static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long long count, long long in_dist,
@@ -451,7 +539,12 @@ static cudaError_t launch_r2c_rows_split(int lm, const float2* in, float2* out, 
     if (group < 1) return cudaErrorInvalidValue;
     for (long long off = 0; off < count; off += group) {
         const long long cnt = count - off < group ? count - off : group;
-        cudaError_t e = launch_cols<false, true>(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
+        bool done;
+        cudaError_t e = launch_real_chain<false>(lm, in + off * in_dist, out + off * out_dist, tmp, cnt, in_dist, out_dist,
+                                                 tw, s, &done);
+        if (e != cudaSuccess) return e;
+        if (done) continue;
+        e = launch_cols<false, true>(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
         if (e == cudaSuccess)
             e = launch_rows_split(p.log2n2, tmp, out + off * out_dist, cnt, p.log2n1, p.log2n1, M, out_dist, tw, s);
         if (e != cudaSuccess) return e;
@@ -529,7 +622,12 @@ static cudaError_t launch_c2r_cols_merge(int lm, const float2* in, float2* out, 
     if (group < 1) return cudaErrorInvalidValue;
     for (long long off = 0; off < count; off += group) {
         const long long cnt = count - off < group ? count - off : group;
-        cudaError_t e = launch_cols_merge(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
+        bool done;
+        cudaError_t e = launch_real_chain<true>(lm, in + off * in_dist, out + off * out_dist, tmp, cnt, in_dist, out_dist,
+                                                tw, s, &done);
+        if (e != cudaSuccess) return e;
+        if (done) continue;
+        e = launch_cols_merge(p.log2n1, in + off * in_dist, tmp, cnt, p.log2n2, in_dist, M, tw, s);
         if (e != cudaSuccess) return e;
         e = launch_rows<true>(p.log2n2, tmp, out + off * out_dist, cnt, p.log2n1, M, out_dist, tw, s);
         if (e != cudaSuccess) return e;
@@ -575,6 +673,15 @@ static cudaError_t attr_cols12()
     return e == cudaSuccess ? cudaFuncSetAttribute(k_cols12<L1, L2, true, false>, a, smem) : e;
 }
 
+template <int LA, int LB>
+static cudaError_t attr_real_chain()
+{
+    const int smem = (int)RealChain<LA, LB>::SMEM;
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_real_chain<LA, LB, false>, a, smem);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k_real_chain<LA, LB, true>, a, smem) : e;
+}
+
 template <int L>
 static cudaError_t attr_pass()
 {
@@ -597,6 +704,10 @@ cudaError_t prepare_large()
     if (e == cudaSuccess) e = attr_pass<8>();
     if (e == cudaSuccess) e = attr_pass<9>();
     if (e == cudaSuccess) e = attr_pass<10>();
+    if (e == cudaSuccess) e = attr_real_chain<8, 9>();
+    if (e == cudaSuccess) e = attr_real_chain<9, 9>();
+    if (e == cudaSuccess) e = attr_real_chain<9, 10>();
+    if (e == cudaSuccess) e = attr_real_chain<10, 10>();
     if (e == cudaSuccess) e = attr_cols12<7, 7>();
     if (e == cudaSuccess) e = attr_cols12<7, 8>();
     if (e == cudaSuccess) e = attr_cols12<8, 8>();
