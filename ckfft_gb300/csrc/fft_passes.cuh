@@ -1,6 +1,7 @@
 // fft_passes.cuh -- the two passes of the multi-pass transform as device
-// functions (used by the batched kernels in fft_large.cu and by the persistent
-// job kernel in fft_jobs.cu).
+// functions, one value a thread and register pair (used by the persistent job
+// kernel in fft_jobs.cu; the batched kernels take the packed passes of
+// fft_pair_passes.cuh, which share the twiddle lookups below).
 //
 // N = N1 * N2, x[n] viewed as N1 rows of N2 columns (n = N2*n1 + n2):
 //   columns: for each column n2, Y[k1] = DFT_N1 over n1 of x[N2*n1 + n2], times
@@ -137,7 +138,7 @@ __device__ __forceinline__ void pass_cols(const float2* __restrict__ in, float2*
 // k = N2 n1 + n2 its partner M - k = N2 (N1 - 1 - n1) + (N2 - n2) is in the
 // same tile (column 0 pairs with itself at row N1 - n1, and with X[M] at
 // row 0).  The tile's raw bins are staged in shared memory and merged into
-// registers (the algebra of merge_elem) before the column DFTs: no merge
+// registers (real_merge) before the column DFTs: no merge
 // pass over HBM.  CG: L2-only loads, as in pass_cols.
 template <int LA, int MAXT = 512, int CMAX = 16, bool CG = false>
 __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2,
@@ -190,84 +191,20 @@ __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, f
     cols_twiddle_store<LA, true, MAXT, CMAX>(v, out, log2n2, n2, t, tw, true);
 }
 
-// Row pass for tile `tile` (rows tile*C .. tile*C+C-1) of one transform.
-// DISCARD: the input is a dead intermediate (scratch) whose L2 lines may be
-// dropped without write-back once read; it must be 128-byte aligned.
-// log2_row_stride: distance between consecutive rows of the input (default:
-// the row length, rows back to back).
-// STREAM: outputs stored with the evict-first hint (false: they are read
-// again soon, by a later phase of the same kernel).
-template <int LB, bool INV, bool CG, int MAXT = 512, bool DISCARD = true, bool STREAM = true, int CMAX = 16>
-__device__ __forceinline__ void pass_rows(const float2* __restrict__ in, float2* __restrict__ out, int log2n1,
-                                          long long tile, int tid, float2* smem, const float2* __restrict__ tw,
-                                          bool live = true, int log2_row_stride = LB)
-{
-    using P = PassCfg<LB, MAXT, CMAX>;
-    constexpr int N2 = 1 << LB;
-    const int r = tid / P::T, t = tid % P::T;
-    const long long n1len = 1ll << log2n1;
-    const long long row0 = tile * P::C;
-    const long long rstride = 1ll << log2_row_stride;
-    const float2* src = in + (row0 + r) * rstride + t;
-    float2 v[P::R];
-#pragma unroll
-    for (int m = 0; m < P::R; ++m) v[m] = live ? ld_data<CG>(src + m * P::T) : make_float2(0.f, 0.f);
-    PaddedView view{smem + r * padded_len(N2)};
-    stockham<LB, P::LOG2R, INV, (P::T <= 32)>(v, t, tw, view);
-    __syncthreads();
-    if (DISCARD && live) {
-        // every thread of the tile has consumed its inputs: the intermediate
-        // rows are dead, so drop their L2 lines instead of writing them back
-        static_assert(N2 % 16 == 0, "rows span whole 128-byte lines");
-        const char* row = (const char*)(in + (row0 + r) * rstride);
-#pragma unroll
-        for (int l = t; l < N2 / 16; l += P::T)
-            asm volatile("discard.global.L2 [%0], 128;" ::"l"(row + 128 * l) : "memory");
-    }
-    // transpose through shared memory so that stores run along rows k1
-#pragma unroll
-    for (int m = 0; m < P::R; ++m) smem[TileView<P::C>::slot(t + m * P::T, r)] = v[m];
-    __syncthreads();
-    if (!live) return;
-    if constexpr (STREAM && P::C % 2 == 0) {
-        if (((uintptr_t)out & 15) == 0) {
-            // two adjacent rows per thread, one 16-byte store each: half the
-            // store instructions (out 16-byte aligned; row0 and r2 even)
-            constexpr int H = P::C / 2, T2 = P::THREADS / H;
-            const int r2 = 2 * (tid % H), t2 = tid / H;
-            float4* dst4 = reinterpret_cast<float4*>(out + row0 + r2);
-#pragma unroll
-            for (int m = 0; m < (1 << LB) / T2; ++m) {
-                const int k2 = t2 + m * T2;
-                const float2 a = smem[TileView<P::C>::slot(k2, r2)], b = smem[TileView<P::C>::slot(k2, r2 + 1)];
-                __stcs(dst4 + (long long)k2 * (n1len / 2), make_float4(a.x, a.y, b.x, b.y));
-            }
-            return;
-        }
-    }
-    const int r2 = tid % P::C, t2 = tid / P::C;
-    float2* dst = out + row0 + r2;
-#pragma unroll
-    for (int m = 0; m < P::R; ++m) {
-        const int k2 = t2 + m * P::T;
-        if constexpr (STREAM) __stcs(dst + (long long)k2 * n1len, smem[TileView<P::C>::slot(k2, r2)]);
-        else dst[(long long)k2 * n1len] = smem[TileView<P::C>::slot(k2, r2)];
-    }
-}
-
 // Row pass with the output transpose folded into the last stage exchange.
 // All stages but the last run on thread (r, t) = (tid / T, tid mod T): row
-// r's positions t + mT, coalesced row loads, exchanges inside the row as in
-// pass_rows.  The second-to-last stage writes its outputs to the row's
+// r's positions t + mT, coalesced row loads, exchanges inside the row.  The second-to-last stage writes its outputs to the row's
 // padded shared-memory image; the last stage then runs on thread
 // (r, t) = (tid mod C, tid / C), so the C lanes of one t hold rows row0 ..
 // row0 + C - 1 and each output store covers C consecutive bins k1 of one
-// k2.  One shared-memory round trip per value fewer than pass_rows
-// (exchange inside the row, then a transpose).  Row images are
+// k2.  One shared-memory round trip per value fewer than an exchange inside
+// the row and a transpose.  Row images are
 // padded_len(N2) slots apart, an odd number: the last stage's reads across
 // 16 rows fall in distinct 8-byte banks.
-// DISCARD / CG / log2_row_stride as in pass_rows; outputs are stored with
-// the evict-first hint.
+// DISCARD: the input is a dead intermediate (scratch) whose L2 lines may be
+// dropped without write-back once read; it must be 128-byte aligned.
+// log2_row_stride: distance between consecutive rows of the input (default:
+// the row length).  Outputs are stored with the evict-first hint.
 template <int LB, bool INV, bool CG, int MAXT = 512, bool DISCARD = true, int CMAX = 16>
 __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, float2* __restrict__ out, int log2n1,
                                              long long tile, int tid, float2* smem, const float2* __restrict__ tw,
@@ -331,12 +268,12 @@ __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, floa
 // are in one CTA.  After the row DFTs the tile's half-length spectrum stays
 // in shared memory and the CTA writes the bins X[k], X[M-k] (M+1 bins per
 // transform) directly: no split pass over HBM.  Same algebra as
-// split_pair_inplace, with the twiddles factored (see below).
+// real_split, with the twiddles factored (see below).
 // The third pass of the three-pass transform is the same pass over
 // N1 = N1' N2' rows: row k1' + N1' k2' sits at in[k1' N2' N3 + k2' N3] (the
 // intermediate of the second pass); log2k1 = log2 N1' selects that address
 // form (log2k1 = log2n1: rows back to back).  CG: L2-only loads, as in
-// pass_rows.
+// pass_cols.
 template <int LB, int MAXT = 512, bool CG = false>
 __device__ __forceinline__ void pass_rows_split(const float2* __restrict__ in, float2* __restrict__ out,
                                                 int log2n1, long long tile, int tid, float2* smem,
@@ -412,35 +349,6 @@ __device__ __forceinline__ void pass_rows_split(const float2* __restrict__ in, f
             out[M - k] = real_split(b, a, make_float2(-w.x, w.y));
         }
     }
-}
-
-// Real forward split, in place: pair k in [0, M/2] of a natural-order
-// half-length spectrum z (room for M+1 values) becomes output bins k and M-k
-// (k = 0 gives bins 0 and M; k = M/2 the middle bin).
-template <bool CG>
-__device__ __forceinline__ void split_pair_inplace(float2* __restrict__ z, long long M, long long k,
-                                                   const float2* __restrict__ twn)
-{
-    if (k == 0) {
-        const float2 z0 = ld_data<CG>(z);
-        z[0] = real_split(z0, z0, __ldg(twn));
-        z[M] = real_split(z0, z0, __ldg(twn + M));
-    } else if (k == M / 2) {
-        const float2 zk = ld_data<CG>(z + k);
-        z[k] = real_split(zk, zk, __ldg(twn + k));
-    } else {
-        const float2 a = ld_data<CG>(z + k), b = ld_data<CG>(z + (M - k));
-        z[k] = real_split(a, b, __ldg(twn + k));
-        z[M - k] = real_split(b, a, __ldg(twn + (M - k)));
-    }
-}
-
-// Real inverse merge of element k < M: y[k] from x[k] and x[M-k].
-template <bool CG>
-__device__ __forceinline__ void merge_elem(const float2* __restrict__ x, float2* __restrict__ y, long long M,
-                                           long long k, const float2* __restrict__ twn)
-{
-    y[k] = real_merge(ld_data<CG>(x + k), ld_data<CG>(x + (M - k)), __ldg(twn + k));
 }
 
 }  // namespace ckg

@@ -82,7 +82,7 @@ struct Slot {
 };
 
 // A direct lane runs one large request at a time through the batched entry
-// points (one launch, or two or three for multi-pass sizes) on its own stream.
+// points (one launch, or several for multi-pass sizes) on its own stream.
 struct Lane {
     Stage stage;
     cudaStream_t stream = nullptr;

@@ -98,7 +98,7 @@ const char* CkFftCudaGetLastError(void);
 /* Batched transforms: `count` independent transforms of size n stored back to
  * back (complex: n values per transform; real forward: n floats in, n/2+1
  * complex out; real inverse: n/2+1 complex in, n floats out).  One kernel
- * launch covers the whole batch (two or three for multi-pass sizes).
+ * launch covers the whole batch (several for multi-pass sizes).
  *
  * stream: a cudaStream_t passed as void*.  With NULL the call blocks until
  * `out` holds the results.  With a stream and device pointers for both `in`
@@ -304,7 +304,7 @@ int CkFftCudaServerReplay(CkFftCudaServer* server, const CkFftCudaRequest* reque
                           double* latency_s, CkFftCudaServeStats* stats);
 
 /* The same trace through the plain path, one batch call per request at its
- * arrival (one launch per request, two or three for multi-pass sizes),
+ * arrival (one launch per request, several for multi-pass sizes),
  * blocking: the comparison point for the server. */
 int CkFftCudaReplayPerRequest(CkFftContext* context, const CkFftCudaRequest* requests, int n,
                               double* latency_s, CkFftCudaServeStats* stats);
