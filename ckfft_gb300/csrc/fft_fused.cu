@@ -105,8 +105,19 @@ k_filter_c2r(const float2* __restrict__ spectra, const float2* __restrict__ filt
     const int g = threadIdx.x / C::T, t = threadIdx.x % C::T;
     const long long f = (long long)blockIdx.x * C::TPB + g;
     const long long fc = f < count ? f : 0;
-    frame_c2r_at<LM>(FilterIn<FILT>{spectra + fc * (M + 1), filter, scale}, RowOut{out + fc * M}, f < count, t,
-                     PaddedView{smem + g * C::SLOT}, tw);
+    const FilterIn<FILT> src{spectra + fc * (M + 1), filter, scale};
+    const PaddedView view{smem + g * C::SLOT};
+    float2 v[C::R];
+    if constexpr (kLoadOnce<C, LM>) c2r_load_once<LM>(src, f < count, t, view, tw, v);
+    else c2r_load<LM>(src, f < count, t, tw, v);
+    stockham<LM, C::LOG2R, true, C::WARP>(v, t, tw, view);
+    // the output's address only now (frame_c2r_at, which holds it from the
+    // start, spills 48 bytes a thread at n = 1024)
+    if (f < count) {
+        const RowOut dst{out + fc * M};
+#pragma unroll
+        for (int m = 0; m < C::R; ++m) dst.st(t + m * C::T, v[m]);
+    }
 }
 
 // Row passes of the generic route.
