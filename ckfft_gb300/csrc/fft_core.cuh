@@ -446,6 +446,28 @@ __device__ __forceinline__ void stockham(float2 (&v)[1 << LOG2R], int t, const f
     }
 }
 
+// The same with the thread at position t1 for the last stage: v[m] = x[t + m*T] in,
+// X[t1 + m*T] out (t1 a permutation of the threads; at least two stages).
+template <int LOG2N, int LOG2R, bool INV, bool WARP, class View>
+__device__ __forceinline__ void stockham(float2 (&v)[1 << LOG2R], int t, int t1, const float2* __restrict__ tw,
+                                         const View& view)
+{
+    using S = Sched<LOG2N, LOG2R>;
+    static_assert(S::nstages >= 2, "a first and a last stage");
+    static_for<0, S::nstages>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        constexpr int lrs = S::lrs(s), lns = S::lns(s);
+        const int ts = s + 1 == S::nstages ? t1 : t;
+        stage_compute<LOG2N, LOG2R, lrs, lns, INV>(v, ts, tw);
+        if constexpr (s + 1 < S::nstages) {
+            stage_write<LOG2N, LOG2R, lrs, lns>(v, ts, view);
+            xsync<WARP>();
+            stage_read<LOG2N, LOG2R>(v, s + 2 == S::nstages ? t1 : t, view);
+            xsync<WARP>();
+        }
+    });
+}
+
 // ------------------------------------------------- real-transform algebra
 // Forward split (real forward, src/ckfft/fft_real_default.cpp:30-58):
 //   X[k] = (z0 + conj z1) - i W_n^k (z0 - conj z1),  z0 = Z[k], z1 = Z[m-k] (Z[m] = Z[0]).

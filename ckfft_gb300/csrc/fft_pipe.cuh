@@ -99,7 +99,7 @@ k_pipe(const float2* __restrict__ in, float2* __restrict__ out, long long ngroup
         const long long f = grp * C::TPB + g;
         if constexpr (KIND == R2C) {
             constexpr int M = N;
-            if constexpr (kMirrorShuffle<C>) {
+            if constexpr (kMirrorWarp<C>) {
                 split_store_warp<C, M>(v, RowOut{out + f * out_dist}, true, t, tw + 2 * M);
             } else {
 #pragma unroll

@@ -133,33 +133,60 @@ __device__ __forceinline__ void split_store(const View& view, const Dst& dst, in
     }
 }
 
-// A frame held by part of a warp (16 or 32 threads, v[m] = position t + m T):
-// position M - (t + m T) is value R - 1 - m of lane T - t (lane 0 mirrors
-// itself: value R - m).  mirror_of(v, m) fetches it, for m >= 1 in lane 0;
-// called by all lanes.
+// Mirrors in registers.  With v[m] = position t + m T, position M - (t + m T) is
+// value R - 1 - m of thread T - t; threads 0 and T/2 mirror themselves (0: value
+// R - m).  A frame inside a warp (16 or 32 threads) fetches it from lane T - t.
+// For the forward split a frame of several warps runs its last stage at
+// positions that put t and T - t in one warp, 16 lanes apart (mirror_pos), so
+// that there too the mirror costs a shuffle of half the values and not a write, a
+// barrier and a read of shared memory: real forward batches of 2^26, us, 2^11
+// 82.6 -> 79.5, 2^12 84.7 -> 80.5, 2^13 93.7 -> 85.8, 2^14 114.9 -> 104.3.  The inverse,
+// whose merge needs both mirrors of a pair at 64 registers, gained nothing from
+// it (2^11 87.8 -> 85.2, 2^12 89.9 -> 91.5, 2^13 99.7 -> 100.6).
 template <class C>
-constexpr bool kMirrorShuffle = C::WARP && (C::T == 16 || C::T == 32) && C::R >= 4;
-template <class C, int M_>
-__device__ __forceinline__ float2 mirror_of(const float2 (&v)[C::R], int t)
+constexpr bool kMirrorWarp = C::WARP && (C::T == 16 || C::T == 32) && C::R >= 4;
+template <class C>
+constexpr bool kMirrorCta = !C::WARP && C::T >= 64 && C::T % 32 == 0 && C::R >= 4;
+template <class C>
+__device__ __forceinline__ int mirror_pos(int t)
 {
-    const float2 a = v[C::R - 1 - M_];
-    float2 b = make_float2(__shfl_sync(0xffffffffu, a.x, (C::T - t) & (C::T - 1), C::T),
-                           __shfl_sync(0xffffffffu, a.y, (C::T - t) & (C::T - 1), C::T));
-    if (t == 0) b = v[M_ == 0 ? 0 : C::R - M_];
-    return b;
+    if constexpr (kMirrorCta<C>) {
+        const int i = (t >> 5) * 16 + (t & 15);
+        return (t & 16) == 0 ? i : i == 0 ? C::T / 2 : C::T - i;
+    } else {
+        return t;
+    }
+}
+// Value a = v[R - 1 - m] of the mirror thread, from the lane mirror_lane names: a
+// thread that mirrors itself names its own, which is the mirror at position T/2
+// and one value off at position 0.  Called by all lanes.
+template <class C>
+__device__ __forceinline__ int mirror_lane(int t)
+{
+    if constexpr (kMirrorCta<C>) return t == 0 ? 0 : t == C::T / 2 ? 16 : (threadIdx.x & 31) ^ 16;
+    else return (C::T - t) & (C::T - 1);
+}
+template <class C>
+__device__ __forceinline__ float2 mirror_xchg(float2 a, int lane)
+{
+    constexpr int W = kMirrorCta<C> ? 32 : C::T;
+    return make_float2(__shfl_sync(0xffffffffu, a.x, lane, W), __shfl_sync(0xffffffffu, a.y, lane, W));
 }
 
-// split_store with the spectrum in the frame's registers (kMirrorShuffle): half
+// split_store with the spectrum in the frame's registers, threads at mirror_pos(..): half
 // the values cross lanes, none go through shared memory.
 template <class C, int M, class Dst>
 __device__ __forceinline__ void split_store_warp(const float2 (&v)[C::R], const Dst& dst, bool live, int t,
                                                  const float2* __restrict__ twn)
 {
     const float2 w0 = __ldg(twn + t);
+    const int ml = mirror_lane<C>(t);
     static_for<0, C::R / 2>([&](auto mc) {
         constexpr int m = decltype(mc)::value;
         const int k = t + m * C::T;
-        const float2 z0 = v[m], z1 = mirror_of<C, m>(v, t);
+        const float2 z0 = v[m];
+        float2 z1 = mirror_xchg<C>(v[C::R - 1 - m], ml);
+        if (t == 0) z1 = v[m == 0 ? 0 : C::R - m];
         const float2 w = split_twiddle<C::R, m, false>(w0, twn, k);
         const float sx = z0.x + z1.x, sy = z0.y - z1.y;
         const float dx = z0.x - z1.x, dy = z0.y + z1.y;
@@ -221,10 +248,15 @@ __device__ __forceinline__ void frame_r2c_at(const Src& src, const Dst& dst, boo
 #pragma unroll
         for (int m = 0; m < C::R; ++m) v[m] = make_float2(0.f, 0.f);
     }
-    stockham<LM, C::LOG2R, false, C::WARP>(v, t, tw, view);
-    if constexpr (kMirrorShuffle<C>) {
+    if constexpr (kMirrorWarp<C>) {
+        stockham<LM, C::LOG2R, false, C::WARP>(v, t, tw, view);
         split_store_warp<C, M>(v, dst, live, t, tw + 2 * M);
+    } else if constexpr (kMirrorCta<C>) {
+        const int t1 = mirror_pos<C>(t);
+        stockham<LM, C::LOG2R, false, C::WARP>(v, t, t1, tw, view);
+        split_store_warp<C, M>(v, dst, live, t1, tw + 2 * M);
     } else {
+        stockham<LM, C::LOG2R, false, C::WARP>(v, t, tw, view);
         // natural-order half-size spectrum Z to shared memory, then split
 #pragma unroll
         for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, v[m]);
@@ -269,7 +301,7 @@ __device__ __forceinline__ void c2r_load(const Src& src, bool live, int t, const
 }
 
 // The same with each bin fetched once and its mirror passed on, across lanes
-// where the frame is in one warp (mirror_of), else through the frame's shared
+// where the frame is in one warp (mirror_xchg), else through the frame's shared
 // memory.  Fetched twice, the second fetch is meant to hit L1 and often does
 // not: 457 MB of L2 reads for 246 MB of traffic in the filter kernel at n =
 // 1024, whose bins are products, formed twice as well.  Measured, batches of
@@ -291,7 +323,7 @@ __device__ __forceinline__ void c2r_load_once(const Src& src, bool live, int t, 
     for (int m = 0; m < C::R; ++m) a[m] = live ? src.ld(t + m * C::T) : make_float2(0.f, 0.f);
     if (live && t == 0) last = src.ld(M);
     const float2 w0 = __ldg(twn + t);
-    if constexpr (!kMirrorShuffle<C>) {
+    if constexpr (!kMirrorWarp<C>) {
 #pragma unroll
         for (int m = 0; m < C::R; ++m) view.st(t + m * C::T, a[m]);
         xsync<C::WARP>();
@@ -300,12 +332,16 @@ __device__ __forceinline__ void c2r_load_once(const Src& src, bool live, int t, 
         constexpr int m = decltype(mc)::value;
         const int p = t + m * C::T;
         float2 b;
-        if constexpr (kMirrorShuffle<C>) b = mirror_of<C, m>(a, t);
-        else b = view.ld((M - p) & (M - 1));
+        if constexpr (kMirrorWarp<C>) {
+            b = mirror_xchg<C>(a[C::R - 1 - m], mirror_lane<C>(t));
+            if (t == 0) b = a[m == 0 ? 0 : C::R - m];
+        } else {
+            b = view.ld((M - p) & (M - 1));
+        }
         if (m == 0 && t == 0) b = last;
         v[m] = real_merge(a[m], b, split_twiddle<C::R, m, false>(w0, twn, p));
     });
-    if constexpr (!kMirrorShuffle<C>) xsync<C::WARP>();
+    if constexpr (!kMirrorWarp<C>) xsync<C::WARP>();
 }
 
 template <int LM, class Src, class Dst, class C = SmallCfg<LM>>
