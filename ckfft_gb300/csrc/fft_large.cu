@@ -355,28 +355,51 @@ static cudaError_t launch_cols12_L(const float2* in, float2* mid, int l3, long l
     return cudaSuccess;
 }
 
-template <bool INV, bool MIRROR>
-static cudaError_t launch_cols12(int l1, int l2, int l3, const float2* in, float2* mid, long long count, long long in_dist,
-                                 const float2* tw, cudaStream_t s)
-{
-    switch (l1 * 16 + l2) {
-    case 7 * 16 + 7: return launch_cols12_L<7, 7, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
-    case 7 * 16 + 8: return launch_cols12_L<7, 8, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
-    case 8 * 16 + 8: return launch_cols12_L<8, 8, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
-    case 8 * 16 + 9: return launch_cols12_L<8, 9, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
-    case 9 * 16 + 9: return launch_cols12_L<9, 9, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
 // Three sub-lengths of at most 2^10 (each >= 2^7), as equal as possible.
-static bool plan3(int log2n, int* l1, int* l2, int* l3)
+static constexpr bool plan3(int log2n, int* l1, int* l2, int* l3)
 {
     if (log2n < 21 || log2n > 30) return false;
     *l3 = (log2n + 2) / 3;
     *l2 = (log2n - *l3 + 1) / 2;
     *l1 = log2n - *l3 - *l2;
     return *l1 >= 7 && *l3 <= 10 && *l2 <= 10;
+}
+
+// The (l1, l2) that plan3 makes of 2^21 .. 2^28, and for real forward transforms of
+// 2^29 packed pairs (n = 2^30; complex sizes end at 2^28).  A panel there is 128 MB
+// and no longer stays in L2: the chain is then two passes like any other.
+#define CKG_COLS12_PAIRS(X) X(7, 7) X(7, 8) X(8, 8) X(8, 9) X(9, 9)
+constexpr int kMaxLog2Half = 29;
+
+static constexpr bool cols12_covers_plan3()
+{
+    for (int log2n = 21; log2n <= kMaxLog2Half; ++log2n) {
+        int l1 = 0, l2 = 0, l3 = 0;
+        if (!plan3(log2n, &l1, &l2, &l3)) return false;
+        bool found = log2n == kMaxLog2Half && l1 == 9 && l2 == 10;
+#define CKG_CASE(L1, L2) found = found || (l1 == L1 && l2 == L2);
+        CKG_COLS12_PAIRS(CKG_CASE)
+#undef CKG_CASE
+        if (!found) return false;
+    }
+    return true;
+}
+static_assert(cols12_covers_plan3(), "every three-pass size has its kernels");
+
+template <bool INV, bool MIRROR>
+static cudaError_t launch_cols12(int l1, int l2, int l3, const float2* in, float2* mid, long long count, long long in_dist,
+                                 const float2* tw, cudaStream_t s)
+{
+    switch (l1 * 16 + l2) {
+#define CKG_CASE(L1, L2) \
+    case L1 * 16 + L2: return launch_cols12_L<L1, L2, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+        CKG_COLS12_PAIRS(CKG_CASE)
+#undef CKG_CASE
+    case 9 * 16 + 10:
+        if constexpr (MIRROR) return launch_cols12_L<9, 10, INV, MIRROR>(in, mid, l3, count, in_dist, tw, s);
+        return cudaErrorInvalidValue;
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 // Sizes from 2^kThreePassMinLog2 on run as three passes whose tiles are all
@@ -708,11 +731,13 @@ cudaError_t prepare_large()
     if (e == cudaSuccess) e = attr_real_chain<9, 9>();
     if (e == cudaSuccess) e = attr_real_chain<9, 10>();
     if (e == cudaSuccess) e = attr_real_chain<10, 10>();
-    if (e == cudaSuccess) e = attr_cols12<7, 7>();
-    if (e == cudaSuccess) e = attr_cols12<7, 8>();
-    if (e == cudaSuccess) e = attr_cols12<8, 8>();
-    if (e == cudaSuccess) e = attr_cols12<8, 9>();
-    if (e == cudaSuccess) e = attr_cols12<9, 9>();
+#define CKG_CASE(L1, L2) \
+    if (e == cudaSuccess) e = attr_cols12<L1, L2>();
+    CKG_COLS12_PAIRS(CKG_CASE)
+#undef CKG_CASE
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_cols12<9, 10, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Cols12<9, 10>::SMEM);
     return e;
 }
 

@@ -58,7 +58,7 @@ __device__ __forceinline__ float2 ld_data(const float2* p)
 
 // W_N^p for 0 <= p < N = 2^ln from two short table levels:
 // W_N^p = W_{N/2^s}^(p >> s) * W_N^(p mod 2^s), s = ceil(ln/2).
-// Sizes on this path are at most 2^28, so p fits in 32 bits.
+// Sizes on this path are at most 2^29, so p fits in 32 bits.
 template <bool INV>
 __device__ __forceinline__ float2 big_twiddle(const float2* __restrict__ tw, int ln, int p)
 {
