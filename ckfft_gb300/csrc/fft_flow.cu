@@ -92,6 +92,7 @@ struct FlowArgs {
     int lag;                   // D
     int* ctl;                  // [0] ticket, [1 + f] finished column tiles of transform f
     unsigned* err;
+    int tries;                 // bound of every wait (kWaitTries)
 };
 
 // Zeroes the ticket and the counters.
@@ -170,12 +171,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 // A bounded wait of one thread for a condition, briefly spinning, then asleep
 // between tries; false (error word set) when it runs out.
 template <class F>
-__device__ __forceinline__ bool flow_wait(F&& ready, unsigned* err)
+__device__ __forceinline__ bool flow_wait(F&& ready, const FlowArgs& a)
 {
 #pragma unroll 1
     for (int tries = 0; !ready(); ++tries) {
-        if (tries == kWaitTries) {
-            if (err) *(volatile unsigned*)err = kErrWaitTimeout;
+        if (tries == a.tries) {
+            if (a.err) *(volatile unsigned*)a.err = kErrWaitTimeout;
             return false;
         }
         __nanosleep(tries > 1000 ? 500 : 20);
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
         if (threadIdx.x % 32 != 0) return;
         int next = atomicAdd(a.ctl, C::kChunk), head = 0;
         auto put = [&](int item) {
-            if (!flow_wait([&] { return min(ld_acquire_cta(&q_tail[0]), ld_acquire_cta(&q_tail[1])) > head - NB; }, a.err))
+            if (!flow_wait([&] { return min(ld_acquire_cta(&q_tail[0]), ld_acquire_cta(&q_tail[1])) > head - NB; }, a))
                 return false;
             queue[head % NB] = item;
             st_release_cta(q_head, ++head);
@@ -278,17 +279,26 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
         // Lane g counts group g's finished column tiles.  The release
         // that makes a tile's stores visible before its count waits for them
         // to reach L2; here that costs the groups nothing.
+        // All lanes stay to the end and leave together: when every group is
+        // through, or after a.tries rounds in which no lane counted anything.
         const int lane = threadIdx.x % 32;
-        int k = 0;
+        int k = 0, quiet = 0;
         bool fin = lane >= G;
 #pragma unroll 1
-        for (int tries = 0; tries < kWaitTries && !__all_sync(0xffffffffu, fin); ++tries) {
+        while (!__all_sync(0xffffffffu, fin)) {
+            bool counted = false;
             if (!fin && mbar_try_wait(done(lane), (uint32_t)k & 1u)) {
                 const int p = sig_f[lane];
                 if (p < 0) fin = true;
                 else red_release(a.ctl + 1 + p);
                 sig_done[lane] = ++k;
-                tries = 0;
+                counted = true;
+            }
+            if (__any_sync(0xffffffffu, counted)) {
+                quiet = 0;
+            } else if (++quiet > a.tries) {
+                if (lane == 0 && a.err) *(volatile unsigned*)a.err = kErrWaitTimeout;
+                return;
             }
         }
         return;
@@ -302,7 +312,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
 #pragma unroll 1
         for (int seq = 0, ends = 0; ends < G; ++seq) {
             const int b = seq % NB;
-            if (!flow_wait([&] { return ld_acquire_cta(q_head) > seq; }, a.err)) return;
+            if (!flow_wait([&] { return ld_acquire_cta(q_head) > seq; }, a)) return;
             const int it = queue[seq % NB];
             bool second = true;
             int f = 0, tile = 0;
@@ -319,8 +329,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
             // wait for the buffer, which covers the latency)
             int have = second && it >= 0 ? ld_acquire(a.ctl + 1 + f) : TA;
             // the group that used the buffer before has read it for the last time
-            if (seq >= NB && !mbar_wait(empty(b), (uint32_t)(seq / NB - 1) & 1u, a.err)) return;
-            if (have < TA && !flow_wait([&] { return ld_acquire(a.ctl + 1 + f) >= TA; }, a.err)) return;
+            if (seq >= NB && !mbar_wait(empty(b), (uint32_t)(seq / NB - 1) & 1u, a.err, a.tries)) return;
+            if (have < TA && !flow_wait([&] { return ld_acquire(a.ctl + 1 + f) >= TA; }, a)) return;
             meta[b].item = it;
             st_release_cta(const_cast<int*>(&meta[b].seq), seq);
             // Only now, and a queue of NB: the other loader is then less than
@@ -353,7 +363,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
     // ------------------------------------------------------------ groups
     const int g = threadIdx.x / GT, tid = threadIdx.x % GT;
     int k = 0;                                          // items given to the counter warp so far
-    // first barrier of an item: false when a thread's wait ran out
+    // first barrier of an item: false when a wait of any of its warps ran out
     auto sync_and = [&](bool ok) {
         int all;
         asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbar.red.and.pred q, %1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
@@ -361,28 +371,42 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
         return all != 0;
     };
     auto sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(GT) : "memory"); };
+    bool ok = true;                                     // none of this thread's waits has run out
+    // The load of use `seq` of its buffer has been started (an earlier use may
+    // still be loading for another group: the phase bit alone cannot tell), and
+    // its data is here.
+    auto landed = [&](int seq) {
+        const int b = seq % NB;
+        return flow_wait([&] { return ld_acquire_cta(const_cast<int*>(&meta[b].seq)) == seq; }, a) &&
+               mbar_wait(full(b), (uint32_t)(seq / NB) & 1u, a.err, a.tries);
+    };
+    // After a wait has run out the group leaves as a whole, at its next
+    // meeting; one thread stays until the loads in flight to the group's buffers
+    // have landed (bounded again).
+    auto leave = [&](int seq) {
+        if (tid == 0)
+            while (landed(seq) && meta[seq % NB].item >= 0) seq += G;
+    };
 #pragma unroll 1
     for (int seq = g;; seq += G) {
         const int b = seq % NB;
-        // The load of this use of the buffer has been started (an earlier use
-        // may still be loading for another group: the phase bit alone cannot
-        // tell), then its data is here.
-        if (!flow_wait([&] { return ld_acquire_cta(const_cast<int*>(&meta[b].seq)) == seq; }, a.err) ||
-            !mbar_wait(full(b), (uint32_t)(seq / NB) & 1u, a.err)) {
-            sync_and(false);                            // the whole group leaves at its next meeting
-            return;
-        }
-        const int it = meta[b].item;
+        // (the warp's answer: its threads take the same way to the barriers)
+        ok = __all_sync(0xffffffffu, ok && landed(seq));
+        const int it = ok ? meta[b].item : -1;
         // a column tile's stores are made: to the counter warp (-1: no more),
         // once it is through with the tile before
         auto finish = [&](int f) {
-            flow_wait([&] { return sig_done[g] >= k; }, a.err);
+            if (!flow_wait([&] { return sig_done[g] >= k; }, a)) {
+                ok = false;
+                return;
+            }
             if (tid == 0) sig_f[g] = f;
             mbar_arrive(done(g));
             ++k;
         };
         if (it < 0) {
-            if (sync_and(true)) finish(-1);
+            if (sync_and(ok)) finish(-1);
+            else leave(seq);
             return;
         }
         cpair* twsm = tws + (2 * g + (k & 1)) * C::TW;
@@ -400,7 +424,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
             const float4* land = reinterpret_cast<const float4*>(buf) + cp;
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = make_pair2(land[(t + m * PA::T) * PA::CP]);
-            if (!sync_and(true)) return;
+            if (!sync_and(ok)) return leave(seq);
             typename PA::ColView view{buf + cp};
             stockham<LA, 4, INV, false>(v, t, tabA, view, sync, [&] { cols_twiddle_put<PA>(twsm, tid, went); }, freed);
             cols_twiddle_store<PA>(v, a.scratch + f * n, LB, n2, cp, t, twsm, wt);
@@ -413,7 +437,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
 #pragma unroll
                 for (int m = 0; m < 16; ++m) v[m] = make_pair2(r0[m * T], r0[N2 + m * T]);
             }
-            if (!sync_and(true)) return;
+            if (!sync_and(ok)) return leave(seq);
             // the bulk copy has read the rows: drop the intermediate's L2 lines
             const char* lines = (const char*)(a.scratch + f * n + ((long long)(tile * PB::C) << LB));
 #pragma unroll
@@ -563,6 +587,7 @@ bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long c
     a.count = (int)count;
     a.ctl = (int*)((char*)scratch + mid);
     a.err = device_error_word();
+    a.tries = kWaitTries;
     switch (log2n) {
     case 17: return launch_flow_L<8, 9>(inverse, a, in, in_dist, s, e);
     case 18: return launch_flow_L<9, 9>(inverse, a, in, in_dist, s, e);
@@ -570,6 +595,29 @@ bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long c
     case 20: return launch_flow_L<10, 10>(inverse, a, in, in_dist, s, e);
     default: return false;
     }
+}
+
+// For the self-test: one CTA starts at the first row tile of one transform none
+// of whose column tiles is ever counted.  Its waits run out after `tries`
+// rounds; no tile is loaded or stored.  `mem`: flow_selftest_bytes(), 128-byte
+// aligned, any contents (it stands for the twiddle table too).
+constexpr size_t kSelftestCtl = sizeof(float2) << 18;
+size_t flow_selftest_bytes() { return kSelftestCtl + 256; }
+cudaError_t launch_flow_selftest(void* mem, int tries, cudaStream_t s)
+{
+    using C = FlowCfg<8, 9>;
+    FlowArgs a = {};
+    a.out = a.scratch = (float2*)mem;
+    a.tw = (const float2*)mem;
+    a.count = a.lag = 1;
+    a.ctl = (int*)((char*)mem + kSelftestCtl);
+    a.err = device_error_word();
+    a.tries = tries;
+    CUtensorMap map;
+    if (!encode_map(&map, mem, 1 << 9, 1 << 8, 1, 1 << 17, C::PA::C)) return cudaErrorNotSupported;
+    const int ctl[2] = {(1 << 9) / C::PA::C, 0};                       // ticket: behind the column tiles
+    const cudaError_t e = cudaMemcpyAsync(a.ctl, ctl, sizeof ctl, cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? launch_pdl(k_flow<8, 9, false>, dim3(1), dim3(kFlowThreads), C::SMEM, s, a, map) : e;
 }
 
 template <int LA, int LB>

@@ -136,6 +136,10 @@ bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long c
                  long long out_dist, const float2* tw, void* scratch, size_t scratch_bytes, cudaStream_t stream,
                  cudaError_t* e);
 
+// One launch of that kernel whose waits run out (selftest.cu).
+size_t flow_selftest_bytes();
+cudaError_t launch_flow_selftest(void* mem, int tries, cudaStream_t stream);
+
 // Complex 2^15 and 2^16 on persistent CTAs, one transform per CTA at a time,
 // both passes inside the CTA with bulk-copied tiles and the intermediate in
 // L2 (fft_mid.cu).  scratch: mid_scratch_bytes(), 128-byte aligned; in

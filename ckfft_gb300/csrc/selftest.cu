@@ -5,7 +5,8 @@
 //
 // Nothing here faults, traps or hangs: the waits are for a condition that
 // nothing ever sets (a job counter no unit increments, an mbarrier expecting
-// bytes no copy delivers), with a short bound, and no copy is ever in flight.
+// bytes no copy delivers, a transform whose column tiles no group finishes), with
+// a short bound, and no copy is ever in flight.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -71,7 +72,8 @@ extern "C" int CkFftCudaSelfTestWait(CkFftContext* context, int which)
 {
     ContextView cv;
     if (!context_view(context, &cv)) return st_fail("NULL or invalid context");
-    if (which != 0 && which != 1) return st_fail("which must be 0 (job counter) or 1 (bulk-copy barrier)");
+    if (which < 0 || which > 2)
+        return st_fail("which must be 0 (job counter), 1 (bulk-copy barrier) or 2 (tile counter of the two-pass queue)");
     int prev = -1;
     cudaGetDevice(&prev);
     if (prev != cv.device && cudaSetDevice(cv.device) != cudaSuccess) return st_fail("cannot select the device");
@@ -106,6 +108,10 @@ extern "C" int CkFftCudaSelfTestWait(CkFftContext* context, int which)
                 a.wait_tries = kSelfTries;
                 e = launch_jobs_one(a, s);
             }
+        } else if (which == 2) {
+            want = kErrWaitTimeout;
+            e = cudaMalloc(&dmem, flow_selftest_bytes());
+            if (e == cudaSuccess) e = launch_flow_selftest(dmem, kSelfTries, s);
         } else {
             want = kErrWaitTimeout;
             k_selftest_mbar<<<1, 32, 0, s>>>(device_error_word(), kSelfTries);
