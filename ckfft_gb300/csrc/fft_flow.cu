@@ -42,6 +42,7 @@
 // Waits are bounded and report through the error word.
 #include <cuda.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "fft_pair_passes.cuh"
@@ -549,6 +550,9 @@ static bool encode_map(CUtensorMap* m, const void* base, long long cols, long lo
 // 106.9, 2^18 x 64 195 -> 172.
 constexpr long long kFlowMinPoints = 3ll << 22;
 
+static std::atomic<long long> g_flow_launches{0};
+extern "C" long long ckg_flow_launches() { return g_flow_launches.load(std::memory_order_relaxed); }
+
 template <int LA, int LB>
 static bool launch_flow_L(bool inverse, FlowArgs a, const void* in, long long in_dist, cudaStream_t s, cudaError_t* e)
 {
@@ -563,7 +567,10 @@ static bool launch_flow_L(bool inverse, FlowArgs a, const void* in, long long in
     if (*e == cudaSuccess)
         *e = inverse ? launch_pdl(k_flow<LA, LB, true>, grid, block, C::SMEM, s, a, map)
                      : launch_pdl(k_flow<LA, LB, false>, grid, block, C::SMEM, s, a, map);
-    if (*e == cudaSuccess) count_launch(2);
+    if (*e == cudaSuccess) {
+        count_launch(2);
+        g_flow_launches.fetch_add(1, std::memory_order_relaxed);
+    }
     return true;
 }
 
@@ -579,6 +586,7 @@ bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long c
     if (count < 1 || (count << log2n) < kFlowMinPoints || ((uintptr_t)scratch & 127)) return false;
     const size_t mid = (sizeof(float2) << log2n) * (size_t)count;
     if (scratch_bytes < mid + flow_scratch_extra(log2n, count)) return false;
+    if (!spans_disjoint(in, in_dist, out, out_dist, count, 1ll << log2n)) return false;
     FlowArgs a = {};
     a.out = (float2*)out;
     a.scratch = (float2*)scratch;

@@ -251,10 +251,7 @@ template <bool INV>
 static cudaError_t launch_real_chain(int lm, const float2* in, float2* out, float2* mid, long long count, long long in_dist,
                                      long long out_dist, const float2* tw, cudaStream_t s, bool* done)
 {
-    const long long n = 1ll << lm;
-    const char *i0 = (const char*)in, *i1 = (const char*)(in + (count - 1) * in_dist + n + 1);
-    const char *o0 = (const char*)out, *o1 = (const char*)(out + (count - 1) * out_dist + n + 1);
-    *done = (count << lm) >= kChainMinPoints && (i1 <= o0 || o1 <= i0);
+    *done = (count << lm) >= kChainMinPoints && spans_disjoint(in, in_dist, out, out_dist, count, (1ll << lm) + 1);
     if (!*done) return cudaSuccess;
     switch (lm) {
     case 17: return launch_real_chain_L<8, 9, INV>(in, out, mid, count, in_dist, out_dist, tw, s);

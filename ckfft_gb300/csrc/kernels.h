@@ -126,16 +126,29 @@ cudaError_t launch_l2pass(int kind, int log2n, const void* in, void* out, long l
                           long long out_dist, const float2* tw, void* scratch, size_t scratch_bytes,
                           cudaStream_t stream);
 
+// Whether `count` transforms of `len` complex values, in_dist apart, and the
+// ranges they write, out_dist apart, have no byte in common.
+inline bool spans_disjoint(const void* in, long long in_dist, const void* out, long long out_dist, long long count,
+                           long long len)
+{
+    const char *i0 = (const char*)in, *i1 = i0 + sizeof(float2) * ((count - 1) * in_dist + len);
+    const char *o0 = (const char*)out, *o1 = o0 + sizeof(float2) * ((count - 1) * out_dist + len);
+    return i1 <= o0 || o1 <= i0;
+}
+
 // Both passes of a batch of complex 2^17 .. 2^20 transforms in one launch with
 // the intermediates in L2 (fft_flow.cu).  False (nothing launched) where it
 // does not apply: other sizes, too little work, data that TMA cannot address
-// (not 16-byte aligned), a scratch block without flow_scratch_extra() bytes
-// behind the intermediates.
+// (not 16-byte aligned), input and output that overlap (two launches read all
+// inputs before the first output, here outputs are written among the loads), a
+// scratch block without flow_scratch_extra() bytes behind the intermediates.
 size_t flow_scratch_extra(int log2n, long long count);
 bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long count, long long in_dist,
                  long long out_dist, const float2* tw, void* scratch, size_t scratch_bytes, cudaStream_t stream,
                  cudaError_t* e);
 
+// Launches of that kernel so far (tests tell the routes apart by it).
+extern "C" long long ckg_flow_launches();
 // One launch of that kernel whose waits run out (selftest.cu).
 size_t flow_selftest_bytes();
 cudaError_t launch_flow_selftest(void* mem, int tries, cudaStream_t stream);
