@@ -104,6 +104,7 @@ static thread_local int t_plain_loads = 0;
 
 PlainLoadsScope::PlainLoadsScope() : prev(t_plain_loads) { t_plain_loads = 1; }
 PlainLoadsScope::~PlainLoadsScope() { t_plain_loads = prev; }
+bool plain_loads_only() { return t_plain_loads != 0; }
 
 int variant_for(Kind kind, int log2c)
 {

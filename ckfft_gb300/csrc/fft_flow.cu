@@ -586,7 +586,7 @@ bool launch_flow(bool inverse, int log2n, const void* in, void* out, long long c
     if (count < 1 || (count << log2n) < kFlowMinPoints || ((uintptr_t)scratch & 127)) return false;
     const size_t mid = (sizeof(float2) << log2n) * (size_t)count;
     if (scratch_bytes < mid + flow_scratch_extra(log2n, count)) return false;
-    if (!spans_disjoint(in, in_dist, out, out_dist, count, 1ll << log2n)) return false;
+    if (plain_loads_only() || !spans_disjoint(in, in_dist, out, out_dist, count, 1ll << log2n)) return false;
     FlowArgs a = {};
     a.out = (float2*)out;
     a.scratch = (float2*)scratch;

@@ -139,7 +139,7 @@ inline bool spans_disjoint(const void* in, long long in_dist, const void* out, l
 // Both passes of a batch of complex 2^17 .. 2^20 transforms in one launch with
 // the intermediates in L2 (fft_flow.cu).  False (nothing launched) where it
 // does not apply: other sizes, too little work, data that TMA cannot address
-// (not 16-byte aligned), input and output that overlap (two launches read all
+// (not 16-byte aligned) or may not (PlainLoadsScope), input and output that overlap (two launches read all
 // inputs before the first output, here outputs are written among the loads), a
 // scratch block without flow_scratch_extra() bytes behind the intermediates.
 size_t flow_scratch_extra(int log2n, long long count);
@@ -224,14 +224,15 @@ int variant_for(Kind kind, int log2c);
 cudaError_t launch_small_shape(Kind kind, int v, int log2c, const void* in, void* out, long long count,
                                long long in_dist, long long out_dist, const float2* tw, cudaStream_t stream,
                                bool* done);
-// While one of these lives on a thread, variant_for() answers 0 on that
-// thread: launches whose input is host memory mapped into the device's
+// While one of these lives on a thread, variant_for() answers 0 on that thread
+// and launch_flow() false: launches whose input is host memory mapped into the device's
 // address space read it with plain loads, never with bulk (TMA) copies.
 struct PlainLoadsScope {
     PlainLoadsScope();
     ~PlainLoadsScope();
     int prev;
 };
+bool plain_loads_only();        // one of them lives on this thread
 // Device word (in mapped host memory) where kernels record a timed-out wait,
 // for the current device; take_device_error() reads and clears it.
 unsigned* device_error_word();
