@@ -1015,6 +1015,7 @@ CkFftContext* CkFftInit(int nMax, CkFftDirection direction, void* buf, size_t* b
     c->pool = new (std::nothrow) LanePool();
     if (!c->pool) { set_error("out of host memory"); goto fail_out; }
     c->magic = kMagic;
+    ckg::pool_user(1);
     return c;
 
 fail_out:
@@ -1031,6 +1032,7 @@ void CkFftShutdown(CkFftContext* c)
         for (Lane* l : c->pool->lanes) free_lane(l);
         delete c->pool;
         cudaFree(c->dtw);
+        ckg::pool_user(-1);
     }
     c->magic = 0;
     if (c->own_buf) std::free(c);

@@ -142,6 +142,41 @@ unsigned take_device_error()
 }
 
 static cudaMemPool_t g_pool[64] = {};
+static unsigned long long g_pool_idle_max[64] = {};
+static int g_pool_users[64] = {};               // open contexts (g_err_mu)
+static std::atomic<long long> g_pool_room[64];  // bytes to ask for before the pool can pass its bound
+static std::mutex g_pool_mu;                    // reuse across streams on, allocate, off
+
+// Pool attributes are refused, and break the capture, while a thread of the
+// process captures a stream in the default mode; not so under this.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static unsigned long long pool_get(cudaMemPool_t pool, cudaMemPoolAttr attr)
+{
+    unsigned long long v = 0;
+    return cudaMemPoolGetAttribute(pool, attr, &v) == cudaSuccess ? v : 0;
+}
+// Bytes the pool holds that no allocation uses (freed in a stream's order,
+// whether or not the stream has come that far).
+static unsigned long long pool_idle(cudaMemPool_t pool)
+{
+    const unsigned long long used = pool_get(pool, cudaMemPoolAttrUsedMemCurrent);
+    const unsigned long long held = pool_get(pool, cudaMemPoolAttrReservedMemCurrent);
+    return held > used ? held - used : 0;
+}
+
+// CKFFT_CUDA_POOL_IDLE_MIB: that bound in MiB; default a sixteenth of the device.
+static unsigned long long idle_max(int dev)
+{
+    if (const char* v = std::getenv("CKFFT_CUDA_POOL_IDLE_MIB"))
+        if (*v) return (unsigned long long)std::strtoull(v, nullptr, 10) << 20;
+    cudaDeviceProp prop;
+    return cudaGetDeviceProperties(&prop, dev) == cudaSuccess ? prop.totalGlobalMem / 16 : 4ull << 30;
+}
 
 static cudaError_t prepare_pool(int dev)
 {
@@ -161,15 +196,42 @@ static cudaError_t prepare_pool(int dev)
     // the pool, but does not ask whether other streams' frees have happened
     // by now: that asking cost a call with an intermediate 15-55 us of host
     // time once a process had used some ten streams (one 2^20 transform pair
-    // on three streams 42-115 us, 13.5 without).
+    // on three streams 42-115 us, 13.5 without).  The price: every live stream
+    // keeps a block of its own until the host waits for its work.  So beyond
+    // idle_max of them pool_alloc_async asks after all.
     int off = 0;
     if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowOpportunistic, &off);
     if (e != cudaSuccess) {
         cudaMemPoolDestroy(pool);
         return e;
     }
+    g_pool_idle_max[dev] = idle_max(dev);
     g_pool[dev] = pool;
     return cudaSuccess;
+}
+
+void pool_give_back(size_t bytes)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !g_pool[dev]) return;
+    RelaxedCapture relaxed;
+    const unsigned long long held = pool_get(g_pool[dev], cudaMemPoolAttrReservedMemCurrent);
+    const unsigned long long keep = held > bytes ? held - bytes : 0;
+    cudaMemPoolTrimTo(g_pool[dev], (size_t)keep);
+    // whole blocks go, and none that would leave less than `keep`
+    if (pool_get(g_pool[dev], cudaMemPoolAttrReservedMemCurrent) > keep) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
+
+void pool_user(int change)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    bool last;
+    {
+        std::lock_guard<std::mutex> lock(g_err_mu);
+        last = (g_pool_users[dev] += change) == 0;
+    }
+    if (last) pool_give_back(~(size_t)0);
 }
 
 // CKFFT_CUDA_FAIL_ALLOC=k: the k-th device allocation the library requests
@@ -206,7 +268,30 @@ cudaError_t pool_alloc_async(void** p, size_t bytes, cudaStream_t s)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64 || !g_pool[dev]) return cudaMallocAsync(p, bytes, s);
-    return cudaMallocFromPoolAsync(p, bytes, g_pool[dev], s);
+    const cudaMemPool_t pool = g_pool[dev];
+    const unsigned long long most = g_pool_idle_max[dev];
+    // a call can grow the pool by no more than it asks for: the attributes are
+    // read only once that much was asked for since the last look
+    bool over = false;
+    if (g_pool_room[dev].fetch_sub((long long)bytes) < (long long)bytes) {
+        RelaxedCapture relaxed;
+        const unsigned long long held = pool_get(pool, cudaMemPoolAttrReservedMemCurrent);
+        g_pool_room[dev].store((long long)most - (long long)held - (long long)bytes);
+        over = held + bytes > most && pool_idle(pool) + bytes > most;
+    }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!over || cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+        return cudaMallocFromPoolAsync(p, bytes, pool, s);        // (a capture's memory is the graph's)
+    // enough lies idle: take over what another stream is through with, and unmap
+    // what is still too much
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    RelaxedCapture relaxed;
+    int on = 1, off = 0;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowOpportunistic, &on);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowOpportunistic, &off);
+    if (pool_idle(pool) > most) cudaMemPoolTrimTo(pool, (size_t)(pool_get(pool, cudaMemPoolAttrUsedMemCurrent) + most));
+    return e;
 }
 
 static cudaError_t prepare_error_word(int dev)

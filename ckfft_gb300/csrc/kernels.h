@@ -239,9 +239,16 @@ unsigned* device_error_word();
 unsigned take_device_error();
 
 // Stream-ordered allocation from a library-owned memory pool on the current
-// device; the pool keeps freed memory (release threshold: unlimited), so
-// repeated calls do not map and unmap device memory.  Free with cudaFreeAsync.
+// device; the pool keeps freed memory, so repeated calls do not map and unmap
+// device memory, and holds at most a sixteenth of the device idle
+// (CKFFT_CUDA_POOL_IDLE_MIB).  Free with cudaFreeAsync.
 cudaError_t pool_alloc_async(void** p, size_t bytes, cudaStream_t s);
+// Unmaps `bytes` (or more: whole blocks) of what lies idle there and no work uses
+// any more, as far as there is that much.
+void pool_give_back(size_t bytes);
+// A context on the current device opens (1) or closes (-1); the last one to
+// close gives back all that is idle.
+void pool_user(int change);
 // cudaMalloc through the library's fault-injection point
 // (CKFFT_CUDA_FAIL_ALLOC=k fails the k-th allocation of the process).
 cudaError_t dev_malloc(void** p, size_t bytes);

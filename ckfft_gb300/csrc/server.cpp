@@ -249,9 +249,16 @@ std::vector<Request> admit(CkFftCudaServer* s, bool* oversized)
         if (!out.empty() && staged + staged_bytes(r) > kStageBytesPerRun) break;
         if (scratch + r.scratch > (long long)s->arena) {
             if (!out.empty()) break;
-            // alone and larger than an arena: admit if free HBM covers it
+            // alone and larger than an arena: admit if free HBM covers it, the
+            // pool's idle blocks given back where it does not
+            const size_t need = (size_t)r.scratch + (256ull << 20);
             size_t free_b = 0, total_b = 0;
-            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || (size_t)r.scratch + (256ull << 20) > free_b) break;
+            cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+            if (e == cudaSuccess && need > free_b) {
+                ckg::pool_give_back(need - free_b);
+                e = cudaMemGetInfo(&free_b, &total_b);
+            }
+            if (e != cudaSuccess || need > free_b) break;
             *oversized = true;
             out.push_back(r);
             s->pending.pop_front();
