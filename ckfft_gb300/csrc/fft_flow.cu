@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
         const int b = seq % NB;
         // (the warp's answer: its threads take the same way to the barriers)
         ok = __all_sync(0xffffffffu, ok && landed(seq));
-        const int it = ok ? meta[b].item : -1;
+        const int it = meta[b].item;
         // a column tile's stores are made: to the counter warp (-1: no more),
         // once it is through with the tile before
         auto finish = [&](int f) {
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
             mbar_arrive(done(g));
             ++k;
         };
-        if (it < 0) {
+        if (it < 0 || !ok) {
             if (sync_and(ok)) finish(-1);
             else leave(seq);
             return;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
             const float4* land = reinterpret_cast<const float4*>(buf) + cp;
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = make_pair2(land[(t + m * PA::T) * PA::CP]);
-            if (!sync_and(ok)) return leave(seq);
+            if (!sync_and(true)) return leave(seq);
             typename PA::ColView view{buf + cp};
             stockham<LA, 4, INV, false>(v, t, tabA, view, sync, [&] { cols_twiddle_put<PA>(twsm, tid, went); }, freed);
             cols_twiddle_store<PA>(v, a.scratch + f * n, LB, n2, cp, t, twsm, wt);
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_flow(const FlowArgs a, cons
 #pragma unroll
                 for (int m = 0; m < 16; ++m) v[m] = make_pair2(r0[m * T], r0[N2 + m * T]);
             }
-            if (!sync_and(ok)) return leave(seq);
+            if (!sync_and(true)) return leave(seq);
             // the bulk copy has read the rows: drop the intermediate's L2 lines
             const char* lines = (const char*)(a.scratch + f * n + ((long long)(tile * PB::C) << LB));
 #pragma unroll
