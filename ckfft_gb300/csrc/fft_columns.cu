@@ -42,13 +42,15 @@ struct ColsCfg {
 
 // Two neighbouring values of a row whose start is not aligned for a pair (an odd
 // number of columns, a base off by one), or with the second (or both) past the
-// last column.  Cached loads: the second finds the first one's sector.
+// last column.  Cached loads: the second finds the first one's sector; not the
+// read-only path, since the kernel ahead may still write the data when this one
+// starts (pdl_wait).
 // (Aligned pairs shifted by one value through the neighbouring lane moved fewer
 // bytes but serialised the loads: complex 2^9 x 30001 65 -> 146 us.)
 __device__ __forceinline__ cpair cols_ld(const float2* p, int live)
 {
-    const float2 a = live > 0 ? __ldg(p) : make_float2(0.f, 0.f);
-    const float2 b = live > 1 ? __ldg(p + 1) : make_float2(0.f, 0.f);
+    const float2 a = live > 0 ? __ldca(p) : make_float2(0.f, 0.f);
+    const float2 b = live > 1 ? __ldca(p + 1) : make_float2(0.f, 0.f);
     return make_pair2(a, b);
 }
 __device__ __forceinline__ void cols_st(float2* p, cpair v, int live)
@@ -59,7 +61,7 @@ __device__ __forceinline__ void cols_st(float2* p, cpair v, int live)
 // The same for neighbouring reals.
 __device__ __forceinline__ f32x2 cols_ld(const float* p, int live)
 {
-    return pack2(live > 0 ? __ldg(p) : 0.f, live > 1 ? __ldg(p + 1) : 0.f);
+    return pack2(live > 0 ? __ldca(p) : 0.f, live > 1 ? __ldca(p + 1) : 0.f);
 }
 __device__ __forceinline__ void cols_st(float* p, f32x2 v, int live)
 {

@@ -54,11 +54,13 @@ __device__ __forceinline__ float2 split_twiddle(float2 w_t, const float2* __rest
 // How a frame body reaches its input and output: element i of a frame (a
 // complex value, or a packed pair of reals on the real side).
 
-// Contiguous rows, streaming loads and stores (the batched layout).
+// Contiguous rows, streaming loads and stores (the batched layout).  ldg: cached
+// for a second read, but not by the read-only path: the kernel ahead in the stream
+// may still write the row when this one starts (pdl_start).
 struct RowIn {
     const float2* __restrict__ p;
     __device__ __forceinline__ float2 ld(long long i) const { return __ldcs(p + i); }
-    __device__ __forceinline__ float2 ldg(long long i) const { return __ldg(p + i); }
+    __device__ __forceinline__ float2 ldg(long long i) const { return __ldca(p + i); }
 };
 struct RowOut {
     float2* __restrict__ p;
