@@ -9,8 +9,8 @@
 // sector per element.  The transforms then run from the slots exactly as in
 // the batched kernels.
 //
-// Where both sides are distance 1, fft_columns.cu takes complex 2^8 .. 2^12 and
-// real n = 2^9 .. 2^13 (all but its smallest sizes where rows are unaligned).
+// Where both sides are distance 1, fft_columns.cu takes complex 2^9 .. 2^12 and
+// real n = 2^10 .. 2^13, and where rows are aligned 2^8 and 2^9.
 //
 // Covered: complex 2^6 .. 2^13 (either side or both interleaved), real
 // forward with interleaved reals, real inverse with interleaved reals, real
@@ -203,6 +203,10 @@ static unsigned inter_grid(long long count)
     return (unsigned)((count + C::G - 1) / C::G);
 }
 
+// Sizes whose distance-1 layouts on both sides come here: the others always go to
+// fft_columns.cu.
+constexpr bool inter_both(int l) { return l <= 8 || l >= 13; }
+
 template <int L, bool INV>
 static cudaError_t launch_c2c_inter_L(const void* in, void* out, long long count, const Layout& lay, bool cin,
                                       bool cout, const float2* tw, cudaStream_t s)
@@ -210,8 +214,10 @@ static cudaError_t launch_c2c_inter_L(const void* in, void* out, long long count
     using C = InterCfg<L>;
     const float2* i = (const float2*)in;
     float2* o = (float2*)out;
-    if (cin && cout) k_c2c_inter<L, INV, true, true><<<inter_grid<C>(count), C::THREADS, C::SMEM, s>>>(i, o, count, lay, tw);
-    else if (cin) k_c2c_inter<L, INV, true, false><<<inter_grid<C>(count), C::THREADS, C::SMEM, s>>>(i, o, count, lay, tw);
+    if (cin && cout) {
+        if constexpr (inter_both(L)) k_c2c_inter<L, INV, true, true><<<inter_grid<C>(count), C::THREADS, C::SMEM, s>>>(i, o, count, lay, tw);
+        else return cudaErrorInvalidValue;
+    } else if (cin) k_c2c_inter<L, INV, true, false><<<inter_grid<C>(count), C::THREADS, C::SMEM, s>>>(i, o, count, lay, tw);
     else k_c2c_inter<L, INV, false, true><<<inter_grid<C>(count), C::THREADS, C::SMEM, s>>>(i, o, count, lay, tw);
     return cudaGetLastError();
 }
@@ -273,10 +279,12 @@ static cudaError_t attr_inter()
     const int smem = (int)InterCfg<L>::SMEM;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, false, true, true>, a, smem);
+    if constexpr (inter_both(L)) {
+        e = cudaFuncSetAttribute(k_c2c_inter<L, false, true, true>, a, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, true, true, true>, a, smem);
+    }
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, false, true, false>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, false, false, true>, a, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, true, true, true>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, true, true, false>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_c2c_inter<L, true, false, true>, a, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_r2c_inter<L>, a, smem);

@@ -9,8 +9,8 @@
 //   rows:    for each row k1, DFT_N2 over n2, X[k1 + N1*k2] stored transposed
 //            through shared memory.
 // A tile is C adjacent columns (or rows), so each warp access covers C*8
-// contiguous bytes.  CG selects L2-only loads (ld.global.cg) for data that
-// another CTA wrote earlier in the same launch.
+// contiguous bytes.  Data loads are L2-only (ld.global.cg): another CTA may have
+// written it earlier in the same launch.
 #pragma once
 #include <cstdint>
 
@@ -19,18 +19,15 @@
 namespace ckg {
 
 // Shape of a sub-transform of 2^LS points inside a pass: R values per thread,
-// C sequences per tile.
-// MAXT: thread budget of the CTA (or CTA subgroup) running the tile.  With
-// 512 threads, sub-lengths above 2^10 take 32 values per thread (128
-// registers); with 1024 threads they keep 16 values (64 registers) and twice
-// the resident warps.
-// CMAX: widest tile (C * 8 bytes per row access).
-template <int LS, int MAXT = 512, int CMAX = 16>
+// C sequences per tile (at most 16: 128 bytes per row access).
+// MAXT: thread budget of the CTA subgroup running the tile.
+template <int LS, int MAXT>
 struct PassCfg {
-    static constexpr int LOG2R = LS < 4 ? LS : (LS <= 10 || MAXT >= 1024) ? 4 : 5;
+    static_assert(LS >= 4 && LS <= 10, "16 values a thread");
+    static constexpr int LOG2R = 4;
     static constexpr int R = 1 << LOG2R;
     static constexpr int T = (1 << LS) / R;
-    static constexpr int C = MAXT / T < CMAX ? MAXT / T : CMAX;
+    static constexpr int C = MAXT / T < 16 ? MAXT / T : 16;
     static constexpr int THREADS = C * T;
     // interleaved (pass 1 and pass-2 transpose) and per-row padded (pass 2) layouts
     static constexpr int INTERLEAVED = (1 << LS) * C + ((1 << LS) * C >> 4) + 1;
@@ -49,13 +46,6 @@ struct TileView {
     __device__ __forceinline__ float2 ld(int pos) const { return base[slot(pos, c)]; }
 };
 
-template <bool CG>
-__device__ __forceinline__ float2 ld_data(const float2* p)
-{
-    if constexpr (CG) return __ldcg(p);
-    else return __ldcs(p);
-}
-
 // W_N^p for 0 <= p < N = 2^ln from two short table levels:
 // W_N^p = W_{N/2^s}^(p >> s) * W_N^(p mod 2^s), s = ceil(ln/2).
 // Sizes on this path are at most 2^29, so p fits in 32 bits.
@@ -72,12 +62,12 @@ __device__ __forceinline__ float2 big_twiddle(const float2* __restrict__ tw, int
 
 // Tail of the column pass: v[m] = Y[k1] of column n2 at k1 = t + m T,
 // multiplied by W_N^(n2 k1) and stored at out[N2 k1 + n2].
-template <int LA, bool INV, int MAXT, int CMAX>
-__device__ __forceinline__ void cols_twiddle_store(float2 (&v)[PassCfg<LA, MAXT, CMAX>::R], float2* __restrict__ out,
+template <int LA, bool INV, int MAXT>
+__device__ __forceinline__ void cols_twiddle_store(float2 (&v)[PassCfg<LA, MAXT>::R], float2* __restrict__ out,
                                                    int log2n2, long long n2, int t, const float2* __restrict__ tw,
                                                    bool live)
 {
-    using P = PassCfg<LA, MAXT, CMAX>;
+    using P = PassCfg<LA, MAXT>;
     const long long n2len = 1ll << log2n2;
     const int ln = LA + log2n2;
     float2* dst = out + n2 + (long long)t * n2len;
@@ -112,12 +102,12 @@ __device__ __forceinline__ void cols_twiddle_store(float2 (&v)[PassCfg<LA, MAXT,
 // Column pass for tile `tile` of one transform, by threads tid = 0..THREADS-1.
 // live == false: the threads take part in the barriers only (no memory
 // access outside the tile's shared memory).
-template <int LA, bool INV, bool CG, int MAXT = 512, int CMAX = 16>
+template <int LA, bool INV, int MAXT>
 __device__ __forceinline__ void pass_cols(const float2* __restrict__ in, float2* __restrict__ out, int log2n2,
                                           long long tile, int tid, float2* smem, const float2* __restrict__ tw,
                                           bool live = true)
 {
-    using P = PassCfg<LA, MAXT, CMAX>;
+    using P = PassCfg<LA, MAXT>;
     const int c = tid % P::C, t = tid / P::C;
     const long long n2len = 1ll << log2n2;
     const long long n2 = tile * P::C + c;
@@ -125,10 +115,10 @@ __device__ __forceinline__ void pass_cols(const float2* __restrict__ in, float2*
     float2 v[P::R];
 #pragma unroll
     for (int m = 0; m < P::R; ++m)
-        v[m] = live ? ld_data<CG>(src + (long long)(t + m * P::T) * n2len) : make_float2(0.f, 0.f);
+        v[m] = live ? __ldcg(src + (long long)(t + m * P::T) * n2len) : make_float2(0.f, 0.f);
     TileView<P::C> view{smem, c};
     stockham<LA, P::LOG2R, INV, false>(v, t, tw, view);
-    cols_twiddle_store<LA, INV, MAXT, CMAX>(v, out, log2n2, n2, t, tw, live);
+    cols_twiddle_store<LA, INV, MAXT>(v, out, log2n2, n2, t, tw, live);
 }
 
 // Column pass of a real inverse transform with the merge fused (M = N1 N2
@@ -139,12 +129,12 @@ __device__ __forceinline__ void pass_cols(const float2* __restrict__ in, float2*
 // same tile (column 0 pairs with itself at row N1 - n1, and with X[M] at
 // row 0).  The tile's raw bins are staged in shared memory and merged into
 // registers (real_merge) before the column DFTs: no merge
-// pass over HBM.  CG: L2-only loads, as in pass_cols.
-template <int LA, int MAXT = 512, int CMAX = 16, bool CG = false>
+// pass over HBM.
+template <int LA, int MAXT>
 __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2,
                                                 long long tile, int tid, float2* smem, const float2* __restrict__ tw)
 {
-    using P = PassCfg<LA, MAXT, CMAX>;
+    using P = PassCfg<LA, MAXT>;
     constexpr int N1 = 1 << LA, H = P::C / 2;
     static_assert(P::C >= 2 && P::C % 2 == 0, "tiles of column pairs");
     const int c = tid % P::C, t = tid / P::C;
@@ -161,9 +151,9 @@ __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, f
 #pragma unroll
     for (int m = 0; m < P::R; ++m) {
         const int n1 = t + m * P::T;
-        smem[TileView<P::C>::slot(n1, c)] = ld_data<CG>(in + (long long)n1 * n2len + n2);
+        smem[TileView<P::C>::slot(n1, c)] = __ldcg(in + (long long)n1 * n2len + n2);
     }
-    const float2 xm = (u == 0 && tid == 0) ? ld_data<CG>(in + M) : make_float2(0.f, 0.f);   // X[M]
+    const float2 xm = (u == 0 && tid == 0) ? __ldcg(in + M) : make_float2(0.f, 0.f);   // X[M]
     __syncthreads();
     // Each thread merges its own elements k = N2 n1 + n2 (rows n1 = t + mT of
     // column n2) into registers, reading the partner X[M - k] from the
@@ -188,7 +178,7 @@ __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, f
     __syncthreads();
     TileView<P::C> view{smem, c};
     stockham<LA, P::LOG2R, true, false>(v, t, tw, view);
-    cols_twiddle_store<LA, true, MAXT, CMAX>(v, out, log2n2, n2, t, tw, true);
+    cols_twiddle_store<LA, true, MAXT>(v, out, log2n2, n2, t, tw, true);
 }
 
 // Row pass with the output transpose folded into the last stage exchange.
@@ -201,16 +191,14 @@ __device__ __forceinline__ void pass_cols_merge(const float2* __restrict__ in, f
 // the row and a transpose.  Row images are
 // padded_len(N2) slots apart, an odd number: the last stage's reads across
 // 16 rows fall in distinct 8-byte banks.
-// DISCARD: the input is a dead intermediate (scratch) whose L2 lines may be
-// dropped without write-back once read; it must be 128-byte aligned.
-// log2_row_stride: distance between consecutive rows of the input (default:
-// the row length).  Outputs are stored with the evict-first hint.
-template <int LB, bool INV, bool CG, int MAXT = 512, bool DISCARD = true, int CMAX = 16>
+// The input is a dead intermediate (scratch, 128-byte aligned) whose L2 lines
+// are dropped without write-back once read.  Outputs are stored with the
+// evict-first hint.
+template <int LB, bool INV, int MAXT>
 __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, float2* __restrict__ out, int log2n1,
-                                             long long tile, int tid, float2* smem, const float2* __restrict__ tw,
-                                             int log2_row_stride = LB)
+                                             long long tile, int tid, float2* smem, const float2* __restrict__ tw)
 {
-    using P = PassCfg<LB, MAXT, CMAX>;
+    using P = PassCfg<LB, MAXT>;
     using S = Sched<LB, P::LOG2R>;
     constexpr int N2 = 1 << LB, R = P::R, T = P::T, LR = P::LOG2R, NST = S::nstages;
     constexpr int RSTRIDE = padded_len(N2);
@@ -218,13 +206,13 @@ __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, floa
     static_assert(RSTRIDE % 2 == 1 && P::C * RSTRIDE <= P::SLOTS, "odd row stride inside the tile's memory");
     const long long n1len = 1ll << log2n1;
     const long long row0 = tile * P::C;
-    const long long rstride = 1ll << log2_row_stride;
+    constexpr long long rstride = N2;
     float2 v[R];
     {
         const int r = tid / T, t = tid % T;
         const float2* src = in + (row0 + r) * rstride + t;
 #pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = ld_data<CG>(src + m * T);
+        for (int m = 0; m < R; ++m) v[m] = __ldcg(src + m * T);
         PaddedView view{smem + r * RSTRIDE};
         static_for<0, NST - 1>([&](auto sc) {
             constexpr int st = decltype(sc)::value;
@@ -234,7 +222,7 @@ __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, floa
         });
     }
     __syncthreads();
-    if constexpr (DISCARD) {
+    {
         // every thread of the tile has consumed its inputs: the intermediate
         // rows are dead, so drop their L2 lines instead of writing them back
         static_assert(N2 % 16 == 0, "rows span whole 128-byte lines");
@@ -269,15 +257,10 @@ __device__ __forceinline__ void pass_rows_xt(const float2* __restrict__ in, floa
 // in shared memory and the CTA writes the bins X[k], X[M-k] (M+1 bins per
 // transform) directly: no split pass over HBM.  Same algebra as
 // real_split, with the twiddles factored (see below).
-// The third pass of the three-pass transform is the same pass over
-// N1 = N1' N2' rows: row k1' + N1' k2' sits at in[k1' N2' N3 + k2' N3] (the
-// intermediate of the second pass); log2k1 = log2 N1' selects that address
-// form (log2k1 = log2n1: rows back to back).  CG: L2-only loads, as in
-// pass_cols.
-template <int LB, int MAXT = 512, bool CG = false>
+template <int LB, int MAXT>
 __device__ __forceinline__ void pass_rows_split(const float2* __restrict__ in, float2* __restrict__ out,
                                                 int log2n1, long long tile, int tid, float2* smem,
-                                                const float2* __restrict__ tw, int log2k1)
+                                                const float2* __restrict__ tw)
 {
     using P = PassCfg<LB, MAXT>;
     constexpr int N2 = 1 << LB, H = P::C / 2;
@@ -291,11 +274,10 @@ __device__ __forceinline__ void pass_rows_split(const float2* __restrict__ in, f
     int k1;
     if (r < H) k1 = u * H + r;
     else k1 = (u == 0 && r == H) ? n1 / 2 : n1 - (u * H + (r - H));
-    const float2* rowp = in + ((long long)(k1 & ((1 << log2k1) - 1)) << (log2n1 - log2k1 + LB)) +
-                         ((long long)(k1 >> log2k1) << LB);
+    const float2* rowp = in + ((long long)k1 << LB);
     float2 v[P::R];
 #pragma unroll
-    for (int m = 0; m < P::R; ++m) v[m] = ld_data<CG>(rowp + t + m * P::T);
+    for (int m = 0; m < P::R; ++m) v[m] = __ldcg(rowp + t + m * P::T);
     PaddedView view{smem + r * padded_len(N2)};
     stockham<LB, P::LOG2R, false, (P::T <= 32)>(v, t, tw, view);
     __syncthreads();
