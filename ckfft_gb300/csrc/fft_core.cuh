@@ -222,18 +222,18 @@ __device__ __forceinline__ void xsync()
 
 // ---------------------------------------- programmatic dependent launch
 // A kernel launched by launch_pdl() may be scheduled while the kernel before
-// it in the stream is still finishing (sm_90+).  Each such kernel calls
-// pdl_start() first: it lets the next kernel begin to launch, then waits
-// until the previous one has completed and its writes are visible, before
-// any memory access.  After a kernel that never signals, the wait returns at
+// it in the stream is still finishing (sm_90+).  Each such kernel lets
+// the next one begin to launch and waits until the previous one has completed and
+// its writes are visible, before it reads or writes data: the single-pass kernels
+// both at once at their start (pdl_start).  After a kernel that never signals, the wait returns at
 // once: the launch then behaves like a plain one.
-// A kernel may split the two to read memory that no kernel writes (the twiddle
-// table) before the wait.
+// The multi-pass and column kernels split the two, and first read memory that no
+// kernel writes (the twiddle table).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel let in only once this one's wait is over: a kernel of few
 // CTAs that runs in one wave then does not share its SMs with the next one's
-// waiting CTAs (one 2^20 transform, two passes: 15.8 -> 10.1 us).
+// waiting CTAs (one 2^20 transform, two passes: 15.8 -> 10.6 us).
 __device__ __forceinline__ void pdl_wait_then_launch()
 {
     pdl_wait();

@@ -54,8 +54,8 @@ namespace ckg {
 constexpr int kFlowComputeThreads = 512;
 constexpr int kFlowThreads = kFlowComputeThreads + 32 * 4;   // scheduler, counter, two loaders
 
-// Columns of 2^LA, rows of 2^LB: groups of 256 threads and 64 KiB tiles (16
-// columns or rows, 8 at 2^10).  Groups of 128 and 32 KiB tiles measured the same
+// Columns of 2^LA, rows of 2^LB: groups of 256 threads and 64 KiB tiles (32
+// columns or rows of 2^8, 16 of 2^9, 8 of 2^10).  Groups of 128 and 32 KiB tiles measured the same
 // at 2^17 and 2^18 and 5-10 % slower above.
 template <int LA, int LB>
 struct FlowCfg {

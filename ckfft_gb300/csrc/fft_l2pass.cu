@@ -89,6 +89,8 @@ k_l2(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict
     const int rank = (int)cg::this_cluster().block_rank();
     const long long f = blockIdx.x / K;
     extern __shared__ __align__(128) cpair smem[];
+    // (the table is read ahead of the wait: it arrives by a copy ahead of all the
+    // grouped launches, and no kernel writes it)
     const float2* x = fr ? fr[f].in : in + f * in_dist;
     float2* y = fr ? fr[f].out : out + f * out_dist;
     float2* s = scratch + f * n;
@@ -102,7 +104,9 @@ k_l2(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict
         else pair_cols<LA, INV, KIND == 2, PA>(x, s, LB, tile, ta, tsm, tw, [] { pdl_wait_then_launch(); });
         __syncthreads();                             // the tile's shared memory is reused
     }
-    // every column tile of the transform is in L2 before any row tile reads it
+    // every column tile of the transform is in L2 before any row tile reads it:
+    // the peers' stores are released by the arrive and acquired by the wait, so
+    // that the row pass's cached loads cannot find older lines
     cluster_barrier();
     // the row pass reloads its twiddles: keeping those it shares with the
     // column pass live across the barrier spills registers

@@ -69,6 +69,10 @@ k_rows(const float2* __restrict__ in, float2* __restrict__ out, int log2n1, long
 // step lets the next one in once its own tiles have passed their waits, so a
 // step's start means that the step before the previous one is complete, and
 // the next step's pass-1 tiles fill this step's tail.
+// A pass-1 tile that does not wait still sees what was written ahead of the call:
+// every CTA of step 0 was through its wait, which completes those kernels, before
+// step 1 could start, and so on; and a kernel starts with no lines in L1, so its
+// loads find nothing older than its start.
 template <int L1, int L2>
 struct Cols12 {
     static constexpr int THREADS = 8 * (1 << ((L1 > L2 ? L1 : L2) - 4));
@@ -176,7 +180,8 @@ k_cols_merge(const float2* __restrict__ in, float2* __restrict__ out, int log2n2
 // launches as in k_cols12: a panel is `per` whole transforms (16 MB of
 // intermediates); step s runs the column pass on panel s, then the row pass on
 // panel s - 1, so the intermediates are read back from L2 and HBM sees the input
-// and the output once.  The column tiles come first: they need no wait, fill
+// and the output once (the column tiles read the caller's input without a wait of
+// their own on the grounds given there).  The column tiles come first: they need no wait, fill
 // the tail of the step before, and by the time the row tiles' turn comes that
 // step is complete (alternating tiles hold half the SMs in their waits: real
 // 2^18 x 127, a forward and an inverse, 226 us on one stream against 199).  Panels
@@ -579,8 +584,8 @@ cudaError_t launch_large_r2c(int log2n, const void* in, void* out, long long cou
 {
     // in: n floats per frame (n/2 packed complex), out: n/2+1 complex per frame
     // (half lengths 2^15 / 2^16: the cluster kernel with the split fused into
-    // its row tiles, 2749 / 2621 GB/s batched at n = 2^16 / 2^17 against 2507
-    // / 2609 for the fused two-pass form through HBM)
+    // its row tiles, 3355 / 3303 GB/s batched at n = 2^16 / 2^17; two launches
+    // through HBM, one value a thread, 2507 / 2609)
     const int lm = log2n - 1;
     const long long M = 1ll << lm;
     if ((uintptr_t)scratch & 127) return cudaErrorInvalidValue;
@@ -662,8 +667,8 @@ cudaError_t launch_large_c2r(int log2n, const void* in, void* out, long long cou
 {
     // in: n/2+1 complex per frame, out: n floats per frame (n/2 packed complex)
     // (half lengths 2^15 / 2^16: the cluster kernel with the merge fused into
-    // its column tiles, 2780 / 2656 GB/s batched at n = 2^16 / 2^17 against
-    // 2714 / 2554 for the fused two-pass form through HBM)
+    // its column tiles, 3347 / 3018 GB/s batched at n = 2^16 / 2^17; two launches
+    // through HBM, one value a thread, 2714 / 2554)
     const int lm = log2n - 1;
     const long long M = 1ll << lm;
     if ((uintptr_t)scratch & 127) return cudaErrorInvalidValue;

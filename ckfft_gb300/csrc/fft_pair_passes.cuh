@@ -1,11 +1,14 @@
 // fft_pair_passes.cuh -- the passes of the multi-pass transform
 // (fft_passes.cuh) with two neighbouring columns or rows per thread in packed
-// FP32 arithmetic (fft_pair.cuh).  Same stages, twiddles and rounding as the
-// one-value passes, so the results are the same bits; a third fewer
+// FP32 arithmetic (fft_pair.cuh).  The complex passes have the stages, twiddles
+// and rounding of the one-value passes, so the same bits (the split and merge
+// passes round their own twiddles, rot32_exact, and mirrored rows and columns in
+// another order: real transforms of a job run, on the one-value passes, differ in the
+// last bits, both within the same error); a third fewer
 // instructions per value (both passes of 2^16: 85 -> 54), and every twiddle
 // load ahead of the data.  With them a pass over more data than L2 runs at the
 // HBM copy rate (2^24 in three passes: 135 -> 120 us, 6.7 TB/s), and the two
-// passes of one 2^20 transform, bound by latency, take 10.1 us instead of 17.1.
+// passes of one 2^20 transform, bound by latency, take 10.6 us instead of 17.1.
 //
 // A tile is CP pairs (C = 2 CP columns or rows).  Loads and stores of
 // neighbouring columns are one 16-byte access where the array allows it, two

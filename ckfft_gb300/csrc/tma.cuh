@@ -1,9 +1,10 @@
 // tma.cuh -- bulk-copy (TMA) and mbarrier helpers, inline PTX for sm_90+ / sm_103a.
 //
-// Only the 1-D bulk form is used (cp.async.bulk global -> shared with an
-// mbarrier completing on the transferred byte count): frames of a batch are
-// contiguous, so one copy moves a whole group of frames.  Copies need 16-byte
-// aligned addresses and a byte count that is a multiple of 16; callers check.
+// The 1-D bulk form (cp.async.bulk global -> shared with an mbarrier completing on
+// the transferred byte count): frames of a batch are contiguous, so one copy moves
+// a whole group of frames.  Copies need 16-byte aligned addresses and a byte count
+// that is a multiple of 16; callers check.  (Column tiles by tensor copies:
+// fft_flow.cu.)
 //
 // Every wait is bounded.  A wait that runs out records kErrWaitTimeout in the
 // error word the kernel was given and returns false; kernels then stop.

@@ -1,6 +1,8 @@
-// tuning_table.h -- generated by ckfft_gb300/autotune.py; do not edit by hand.
-// Measured on NVIDIA GB300, 2026-12-04; rinv 7 and 9 .. 11 again on 2026-12-05,
-// when the plain kernels had come to fetch each bin once.
+// tuning_table.h -- generated by ckfft_gb300/autotune.py, measured on NVIDIA GB300,
+// 2026-12-04; then rinv 7 and 9 .. 11 set by hand from a measurement of 2026-12-05,
+// when the plain kernels had come to fetch each bin once (batches of 2^26 reals, us,
+// tuned before / now: 2^8 87.0 / 85.5, 2^10 87.9 / 83.2, 2^11 92.6 / 87.8, 2^12 94.5 /
+// 90.4).  Running the tuner writes the whole table anew.
 // kTunedLog2R[L]: values per thread (log2) of every single-CTA kernel family
 // (batched, pipelined, strided, fused, grouped, job kernel) for complex
 // (half-)length 2^L, so that all of them compute a size with the same radices.
